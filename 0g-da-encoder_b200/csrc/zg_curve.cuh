@@ -19,8 +19,7 @@ namespace zg {
 //   MulImad   both products of a pair on the integer multiply-add pipe
 //             (Fq::mul2, the two CIOS carry chains interleaved);
 //   MulHybrid the first on the integer pipe (Fq::mul), the second on the FP64
-//             pipe (f52::mont_mul): the MSM bucket loop saturates the integer
-//             pipe with carry-chain IMADs, so this pair keeps both pipes busy;
+//             pipe (f51::mont_mul), so both pipes are busy;
 //   MulF64    both on the FP64 pipe;
 //   MulW28    both as 28-bit-limb products with 64-bit column sums
 //             (w28::mont_mul: wide multiply-adds without carry flags, the
@@ -44,10 +43,10 @@ static __device__ __noinline__ FqPair fq_mul2_imad_ool(const Fq a, const Fq b, c
 static __device__ __noinline__ FqPair fq_mul2_hybrid_ool(const Fq a, const Fq b, const Fq c, const Fq d) {
   FqPair r;
   r.a = Fq::mul(a, b);
-  r.b = f52::mont_mul(c, d);
+  r.b = f51::mont_mul(c, d);
   return r;
 }
-static __device__ __noinline__ Fq fq_mul_f64_ool(const Fq a, const Fq b) { return f52::mont_mul(a, b); }
+static __device__ __noinline__ Fq fq_mul_f64_ool(const Fq a, const Fq b) { return f51::mont_mul(a, b); }
 static __device__ __noinline__ Fq fq_mul_w28_ool(const Fq a, const Fq b) { return w28::mont_mul(a, b); }
 static __device__ __noinline__ FqPair fq_mul2_w28_ool(const Fq a, const Fq b, const Fq c, const Fq d) {
   FqPair r;
@@ -58,13 +57,13 @@ static __device__ __noinline__ FqPair fq_mul2_w28_ool(const Fq a, const Fq b, co
 static __device__ __noinline__ FqPair fq_mul2_w28f64_ool(const Fq a, const Fq b, const Fq c, const Fq d) {
   FqPair r;
   r.a = w28::mont_mul(a, b);
-  r.b = f52::mont_mul(c, d);
+  r.b = f51::mont_mul(c, d);
   return r;
 }
 static __device__ __noinline__ FqPair fq_mul2_f64_ool(const Fq a, const Fq b, const Fq c, const Fq d) {
   FqPair r;
-  r.a = f52::mont_mul(a, b);
-  r.b = f52::mont_mul(c, d);
+  r.a = f51::mont_mul(a, b);
+  r.b = f51::mont_mul(c, d);
   return r;
 }
 struct MulImad {
