@@ -260,9 +260,8 @@ struct Lane {
     uint32_t* ents = nullptr;   // [cap][3][units][W 2^ulog]
   };
   std::vector<Wd> wd;           // per wide class of the context
-  XYZZ* fb_T = nullptr;         // [cap][items][FB_ACC_THREADS]
-  XYZZ* fb_S = nullptr;
-  XYZZ* fb_gbuf = nullptr;      // per persistent CTA task partial sums
+  G1Aff* fb_out = nullptr;      // [cap][items][FB_OUT] row and column sums of the bucket grids
+  FbScratch fb_scratch;         // k_fb_accum's scratch, one block per persistent CTA
   uint32_t* fb_next = nullptr;  // k_fb_accum's item counter
   XYZZ* win = nullptr;          // 8-bit path: [3][L][R][MSM_WINDOWS] (cap 1)
   XYZZ* part = nullptr;         // [cap][3][L][R] per-item MSM results
@@ -491,6 +490,14 @@ uint32_t blob_items(const zg_ctx* c) {
   return u;
 }
 
+// k_fb_accum's segment size: the entries of a group of a context's largest
+// items, with half as many again for a wide unit's block 0
+uint32_t fb_segment(const zg_ctx* c) {
+  uint32_t n = (uint32_t)(FB_WINDOWS * c->C);
+  for (const zg_ctx::WdClass& k : c->wd) n = std::max(n, ((uint32_t)wd_windows(k.ulog) * 1536u) << k.mlog);
+  return (uint32_t)FB_GROUP * std::min(n, FB_CAP_MAX);
+}
+
 // device bytes of a lane of `cap` blob slots (the request pipeline's
 // admission compares this with the free HBM)
 size_t lane_bytes(const zg_ctx* c, int cap) {
@@ -499,13 +506,13 @@ size_t lane_bytes(const zg_ctx* c, int cap) {
   size_t per = 3 * (size_t)c->L * R * sizeof(XYZZ) + 3 * (4 * R - 2) * sizeof(XYZZ);
   if (c->fb) {
     per += 3 * R * (FB_BUCKETS + 1) * 4 + 3 * R * FB_WINDOWS * c->C * 2 +
-           2 * (size_t)blob_items_max(c) * FB_ACC_THREADS * sizeof(XYZZ);
+           (size_t)blob_items_max(c) * FB_OUT * sizeof(G1Aff);
     for (size_t j = 0; j < c->wd.size(); ++j) {
       const zg_ctx::WdClass& k = c->wd[j];
       if (k.sort_of == (int)j)
         per += 3 * (N >> k.ulog) * (((size_t)1 << k.ulog) + 1) * 4 + 3 * (N >> k.ulog) * wd_unit_ents(k.ulog) * 4;
     }
-    b += (size_t)c->fb_ctas_max() * FB_MAX_TASKS * sizeof(XYZZ);
+    b += (size_t)c->fb_ctas_max() * FbScratch{nullptr, fb_segment(c)}.bytes();
   } else {
     per += 3 * (size_t)c->L * R * MSM_WINDOWS * sizeof(XYZZ);
   }
@@ -513,7 +520,7 @@ size_t lane_bytes(const zg_ctx* c, int cap) {
 }
 
 void free_lane(Lane* ln) {
-  void* ps[] = {ln->T1, ln->Bc, ln->fb_offs, ln->fb_ents, ln->fb_T, ln->fb_S, ln->fb_gbuf, ln->fb_next,
+  void* ps[] = {ln->T1, ln->Bc, ln->fb_offs, ln->fb_ents, ln->fb_out, ln->fb_scratch.base, ln->fb_next,
                 ln->win, ln->part, ln->nodes};
   for (void* p : ps) if (p) cudaFree(p);
   for (Lane::Wd& w : ln->wd) {
@@ -533,8 +540,7 @@ int alloc_lane(zg_ctx* c, Lane* ln, int cap) {
   if (c->fb) {
     ZG_CK(cudaMalloc(&ln->fb_offs, k * 3 * R * (FB_BUCKETS + 1) * sizeof(uint32_t)));
     ZG_CK(cudaMalloc(&ln->fb_ents, k * 3 * R * FB_WINDOWS * c->C * sizeof(uint16_t)));
-    ZG_CK(cudaMalloc(&ln->fb_T, k * blob_items_max(c) * FB_ACC_THREADS * sizeof(XYZZ)));
-    ZG_CK(cudaMalloc(&ln->fb_S, k * blob_items_max(c) * FB_ACC_THREADS * sizeof(XYZZ)));
+    ZG_CK(cudaMalloc(&ln->fb_out, k * blob_items_max(c) * FB_OUT * sizeof(G1Aff)));
     ln->wd.resize(c->wd.size());
     for (size_t j = 0; j < c->wd.size(); ++j) {
       if (c->wd[j].sort_of != (int)j) continue;  // reads another class's sort output
@@ -542,7 +548,8 @@ int alloc_lane(zg_ctx* c, Lane* ln, int cap) {
       ZG_CK(cudaMalloc(&ln->wd[j].offs, k * 3 * units * (((size_t)1 << c->wd[j].ulog) + 1) * sizeof(uint32_t)));
       ZG_CK(cudaMalloc(&ln->wd[j].ents, k * 3 * units * wd_unit_ents(c->wd[j].ulog) * sizeof(uint32_t)));
     }
-    ZG_CK(cudaMalloc(&ln->fb_gbuf, (size_t)c->fb_ctas_max() * FB_MAX_TASKS * sizeof(XYZZ)));
+    ln->fb_scratch.cap = fb_segment(c);
+    ZG_CK(cudaMalloc(&ln->fb_scratch.base, (size_t)c->fb_ctas_max() * ln->fb_scratch.bytes()));
     ZG_CK(cudaMalloc(&ln->fb_next, sizeof(uint32_t)));
   } else {
     ZG_CK(cudaMalloc(&ln->win, 3 * (size_t)c->L * R * MSM_WINDOWS * sizeof(XYZZ)));
@@ -802,8 +809,7 @@ FbAccArgs blob_fb_args(const zg_ctx* c, const Lane& ln, int b = 0) {
   fa.tab = c->tab;
   fa.offs = ln.fb_offs + (size_t)b * 3 * R * (FB_BUCKETS + 1);
   fa.ents = ln.fb_ents + (size_t)b * 3 * R * FB_WINDOWS * c->C;
-  fa.outT = ln.fb_T + (size_t)b * blob_items(c) * FB_ACC_THREADS;
-  fa.outS = ln.fb_S + (size_t)b * blob_items(c) * FB_ACC_THREADS;
+  fa.out = ln.fb_out + (size_t)b * blob_items(c) * FB_OUT;
   fa.lr = c->lr;
   fa.lc = c->lc;
   fa.lines = c->n_lines;
@@ -815,7 +821,7 @@ FbAccArgs blob_fb_args(const zg_ctx* c, const Lane& ln, int b = 0) {
 }
 
 // first item of wide class k in a blob's item order (chunk items, then the
-// classes); the (T, S) partials of item u sit at fb_T / fb_S + 128 u
+// classes); the sums of item u sit at fb_out + FB_OUT u
 uint32_t blob_wd_first_item(const zg_ctx* c, size_t k) {
   uint32_t u = (uint32_t)(3 * c->R * c->n_lines);
   for (size_t j = 0; j < k; ++j) u += (uint32_t)(3 * (c->R >> c->wd[j].mlog) * c->wd[j].nl);
@@ -834,13 +840,12 @@ uint32_t* lane_wd_ents(const zg_ctx* c, const Lane& ln, size_t k, int b) {
 // blob slot b's work items of wide class k: (coset, unit block, line)
 FbAccArgs blob_wd_args(const zg_ctx* c, const Lane& ln, size_t k, int b = 0) {
   const zg_ctx::WdClass& w = c->wd[k];
-  const size_t first = ((size_t)b * blob_items(c) + blob_wd_first_item(c, k)) * FB_ACC_THREADS;
+  const size_t first = ((size_t)b * blob_items(c) + blob_wd_first_item(c, k)) * FB_OUT;
   FbAccArgs fa;
   fa.tab = w.tab;
   fa.offs = lane_wd_offs(c, ln, k, b);
   fa.ents32 = lane_wd_ents(c, ln, k, b);
-  fa.outT = ln.fb_T + first;
-  fa.outS = ln.fb_S + first;
+  fa.out = ln.fb_out + first;
   fa.lr = c->lr - w.mlog;  // 2^lr items per (coset, line)
   fa.lc = c->lc;
   fa.lines = w.nl;
@@ -901,17 +906,19 @@ __global__ void k_fill_payload(uint8_t* p, uint64_t n, uint64_t seed) {
 // counter and task scratch
 void launch_fb_accum(const zg_ctx* c, const Lane& ln, uint32_t kind, const FbAccPlan& p, cudaStream_t s) {
   const uint32_t units = p.start[p.n];
-  const unsigned grid = std::min<unsigned>(c->fb_ctas[kind], units);
+  // two items per CTA and turn once every resident CTA has that many
+  const uint32_t group = units >= 2 * c->fb_ctas[kind] ? FB_GROUP : 1;
+  const unsigned grid = std::min<unsigned>(c->fb_ctas[kind], (units + group - 1) / group);
   cudaMemsetAsync(ln.fb_next, 0, sizeof(uint32_t), s);
-  const uint32_t task = c->msm_task;
+  auto go = [&](auto kernel) {
+    kernel<<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_scratch, ln.fb_next, c->msm_task, group);
+  };
   switch (kind) {
-    case ZG_MSM_PRODUCT_IMAD: k_fb_accum<MulImad><<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_gbuf, ln.fb_next, task); break;
-    case ZG_MSM_PRODUCT_FP64: k_fb_accum<MulF64><<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_gbuf, ln.fb_next, task); break;
-    case ZG_MSM_PRODUCT_W28: k_fb_accum<MulW28><<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_gbuf, ln.fb_next, task); break;
-    case ZG_MSM_PRODUCT_W28_HYBRID:
-      k_fb_accum<MulW28Hybrid><<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_gbuf, ln.fb_next, task);
-      break;
-    default: k_fb_accum<MulHybrid><<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_gbuf, ln.fb_next, task); break;
+    case ZG_MSM_PRODUCT_IMAD: go(k_fb_accum<MulImad>); break;
+    case ZG_MSM_PRODUCT_FP64: go(k_fb_accum<MulF64>); break;
+    case ZG_MSM_PRODUCT_W28: go(k_fb_accum<MulW28>); break;
+    case ZG_MSM_PRODUCT_W28_HYBRID: go(k_fb_accum<MulW28Hybrid>); break;
+    default: go(k_fb_accum<MulHybrid>); break;
   }
 }
 
@@ -959,12 +966,12 @@ FbAccPlan blob_acc_plan(const zg_ctx* c, const Lane& ln, int nb = 1) {
   return p;
 }
 
-// P = sum_i T_i + 8 sum_i i S_i per item: one thread per item for a blob's
+// the items' results from their grid sums: one thread per item for a blob's
 // items (fewest additions), one warp per item below 16 384 items
 void launch_fb_combine(const Lane& ln, const FbCombinePlan& p, cudaStream_t s) {
   const uint32_t units = p.start[p.n];
-  if (units >= 16384) k_fb_combine<<<nblk(units, 64), 64, 0, s>>>(ln.fb_T, ln.fb_S, ln.part, p);
-  else k_fb_combine_warp<<<nblk((size_t)units * 32, 128), 128, 0, s>>>(ln.fb_T, ln.fb_S, ln.part, p);
+  if (units >= 16384) k_fb_combine<<<nblk(units, 64), 64, 0, s>>>(ln.fb_out, ln.part, p);
+  else k_fb_combine_warp<<<nblk((size_t)units * 32, 128), 128, 0, s>>>(ln.fb_out, ln.part, p);
 }
 
 // k_wd_sort / k_wd_tables for a class's unit size
@@ -1991,8 +1998,7 @@ int verify_msms(VerifyRun& v, const bool present[3], XYZZ* out) {
     fa.tab = c->line_ptr(cs, c->lr);
     fa.offs = c->lane.fb_offs;
     fa.ents = c->lane.fb_ents;
-    fa.outT = c->lane.fb_T;
-    fa.outS = c->lane.fb_S;
+    fa.out = c->lane.fb_out;
     fa.ents32 = nullptr;
     fa.lr = c->lr;
     fa.lc = c->lc;
@@ -3133,8 +3139,7 @@ int zg_ctx_msm(zg_ctx* c, uint32_t coset, uint32_t line, const void* d_scalars, 
   fa.tab = c->line_ptr((int)coset, (int)line);
   fa.offs = c->lane.fb_offs;
   fa.ents = c->lane.fb_ents;
-  fa.outT = c->lane.fb_T;
-  fa.outS = c->lane.fb_S;
+  fa.out = c->lane.fb_out;
   fa.ents32 = nullptr;
   fa.lr = lrn;
   fa.lc = lcs;

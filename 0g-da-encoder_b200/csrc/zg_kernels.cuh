@@ -490,9 +490,7 @@ constexpr int FB_BITS = 11;
 constexpr int FB_WINDOWS = 24;                    // ceil((254 + 1) / 11)
 constexpr int FB_BUCKETS = 1 << (FB_BITS - 1);    // 1024
 constexpr int FB_ACC_THREADS = 128;
-constexpr int FB_PER_THREAD = FB_BUCKETS / FB_ACC_THREADS;  // 8 buckets per thread
 __host__ __device__ constexpr int fb_log2(int x) { return x <= 1 ? 0 : 1 + fb_log2(x / 2); }
-constexpr int FB_PER_THREAD_LOG = fb_log2(FB_PER_THREAD);
 constexpr int FB_ACC_MIN_CTAS = 512 / FB_ACC_THREADS;  // resident CTAs per SM at 128 registers
 
 // Wide windows for the AMT lines whose nodes are MSMs over more than 1024
@@ -761,219 +759,9 @@ __global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __re
   }
 }
 
-struct FbAccArgs {
-  const G1Aff* tab = nullptr;      // [cosets][Ltot][W][tabN]
-  const uint32_t* offs = nullptr;
-  const uint16_t* ents = nullptr;    // chunk items
-  const uint32_t* ents32 = nullptr;  // wide items (k_wd_sort's lists)
-  XYZZ* outT = nullptr;            // [cosets * nchunks * lines][FB_ACC_THREADS]
-  XYZZ* outS = nullptr;
-  int lr = 0, lc = 0, lines = 1;   // 2^lr items of each of `lines` lines per coset
-  int l0 = 0, Ltot = 1;            // item line l reads table line l0 + l of Ltot per coset
-  int ulog = 10;                   // wide items: sort units of 2^ulog points
-  int mlog = 0;                    // wide items: 2^mlog consecutive sort units share buckets
-  int W = FB_WINDOWS;              // windows per table line (wd_windows(ulog) for wide items)
-  uint64_t tabN = 0;               // points per window table (the param line length)
-};
-
-// Persistent CTAs over the (chunk, line) work items. Per item:
-//  1. every bucket is cut into tasks of at most tsz entries (the top
-//     window's digits are tiny, so buckets 1 and 2 hold ~10x the average);
-//     tsz = task unless the item holds more than (FB_MAX_TASKS -
-//     FB_BUCKETS) * task entries (wide items of skewed scalars), so an
-//     item never has more than FB_MAX_TASKS tasks;
-//  2. tasks are counting-sorted by size and round r gives thread i the task at
-//     sorted position 128 r + i: the 32 lanes of a warp run tasks of nearly
-//     equal length;
-//  3. task partial sums go to this CTA's scratch (gpart, L2-resident);
-//  4. thread i merges the partials of buckets 8i+1 .. 8i+8 and folds them
-//     into running sums S_i = sum B_k, T_i = sum (k - 8i) B_k.
-// Wide items (ents32 set) are 1024-bucket blocks of a wide unit of 2^(ulog +
-// mlog) points whose buckets are those of its 2^mlog sort units of 2^ulog
-// points (k_wd_sort; mlog <= 1): item g of a coset is block g & (2^(ulog -
-// 10) - 1) of unit g >> (ulog - 10); bucket k's entries are those of sort
-// unit 0 followed by those of sort unit 1, indexing the points of the
-// merged unit and the W windows of the wide table. A merged unit pays one
-// bucket reduction for twice the points.
-// One launch covers up to FB_MAX_SETS item sets (a blob's chunk items and its
-// wide classes, for up to FB_MAX_BLOBS blobs whose MSMs share the launch):
-// set k holds items start[k] .. start[k + 1] - 1, described by a[k] with
-// local item index u - start[k]. One launch keeps the persistent CTAs busy to
-// the end of the whole MSM instead of leaving a partial last round per set. A CTA takes its next item from the counter *next (zero at
-// launch): items differ in size (a wide unit's block 0 holds the top
-// window's digits), and a fixed item-to-CTA map would give some CTAs every
-// heavy item.
-constexpr int FB_MAX_BLOBS = 2;  // blobs per fused MSM launch
-constexpr int FB_MAX_SETS = 8 * FB_MAX_BLOBS;
-struct FbAccPlan {
-  int n = 0;
-  uint32_t start[FB_MAX_SETS + 1] = {};
-  FbAccArgs a[FB_MAX_SETS];
-};
-// Bucket task size (entries per task, a tuning choice within [FB_TASK_MIN,
-// FB_TASK_MAX]); the task arrays are sized for the smallest.
-constexpr int FB_TASK_MIN = 32;
-constexpr int FB_TASK_MAX = 96;
-constexpr int FB_TASK_DEFAULT = 64;
-constexpr int FB_MAX_TASKS = FB_BUCKETS + FB_WINDOWS * 1024 / FB_TASK_MIN;  // chunk <= 1024 points
-// M is the product kind of the point additions (MulImad / MulHybrid / MulF64,
-// chosen by the context's tuning; identical results).
-template <class M>
-__global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS) k_fb_accum(const FbAccPlan plan, XYZZ* __restrict__ gpart_all,
-                                                                uint32_t* __restrict__ next, uint32_t task) {
-  __shared__ uint32_t soffs[FB_BUCKETS + 1];
-  __shared__ uint32_t soffs2[FB_BUCKETS + 1];  // the second sort unit of a merged wide item
-  __shared__ uint16_t tstart[FB_BUCKETS + 1];
-  __shared__ uint16_t order[FB_MAX_TASKS];
-  __shared__ uint16_t tbucket[FB_MAX_TASKS];
-  __shared__ uint32_t bins[FB_TASK_MAX + 1];
-  task = min(max(task, (uint32_t)FB_TASK_MIN), (uint32_t)FB_TASK_MAX);
-  __shared__ uint32_t item;
-  XYZZ* gpart = gpart_all + (size_t)blockIdx.x * FB_MAX_TASKS;
-  const uint32_t units = plan.start[plan.n];
-  for (;;) {
-    __syncthreads();  // every thread has read the previous item number
-    if (threadIdx.x == 0) item = atomicAdd(next, 1u);
-    __syncthreads();
-    const uint32_t gu = item;
-    if (gu >= units) break;
-    int set = 0;
-    while (set + 1 < plan.n && gu >= plan.start[set + 1]) ++set;
-    const FbAccArgs& a = plan.a[set];
-    const uint32_t u = gu - plan.start[set];
-    const uint32_t nch = 1u << a.lr;
-    const uint64_t N = a.tabN;
-    const uint32_t l = u % a.lines, g = u / a.lines;
-    const uint32_t coset = g / nch, b = g % nch;
-    const uint32_t* offs;
-    const uint32_t* offs2 = nullptr;
-    const uint16_t* ents = nullptr;
-    const uint32_t* ents32 = a.ents32;
-    const uint32_t* ents32b = nullptr;
-    const bool wide = ents32 != nullptr;
-    const uint32_t ulog = (uint32_t)a.ulog;
-    const G1Aff* tabl;
-    if (wide) {
-      const int bl = a.ulog - 10, ml = a.mlog;
-      const uint32_t unit = b >> bl, blk = b & ((1u << bl) - 1);
-      const size_t cu = (size_t)coset * ((size_t)(nch >> bl) << ml) + ((size_t)unit << ml);  // first sort unit
-      offs = a.offs + cu * ((1u << a.ulog) + 1) + (size_t)blk * FB_BUCKETS;
-      ents32 += cu * wd_unit_ents(a.ulog);
-      if (ml) {
-        offs2 = offs + ((1u << a.ulog) + 1);
-        ents32b = ents32 + wd_unit_ents(a.ulog);
-      }
-      tabl = a.tab + ((uint64_t)coset * a.Ltot + a.l0 + l) * a.W * N + ((uint64_t)unit << (a.ulog + ml));
-    } else {
-      offs = a.offs + (size_t)g * (FB_BUCKETS + 1);
-      ents = a.ents + (size_t)g * FB_WINDOWS * (1u << a.lc);
-      tabl = a.tab + ((uint64_t)coset * a.Ltot + a.l0 + l) * FB_WINDOWS * N + ((uint64_t)b << a.lc);
-    }
-    __syncthreads();  // the previous item is finished with the shared arrays and gpart
-    for (int k = threadIdx.x; k <= FB_BUCKETS; k += blockDim.x) {
-      soffs[k] = offs[k];
-      soffs2[k] = offs2 ? offs2[k] : 0u;
-    }
-    for (int k = threadIdx.x; k <= FB_TASK_MAX; k += blockDim.x) bins[k] = 0;
-    __syncthreads();
-    // entries of bucket k (0-based): its range in the first sort unit's list,
-    // then (merged items) its range in the second's
-    auto bcount = [&](int k) { return (soffs[k + 1] - soffs[k]) + (soffs2[k + 1] - soffs2[k]); };
-    const uint32_t nent = (soffs[FB_BUCKETS] - soffs[0]) + (soffs2[FB_BUCKETS] - soffs2[0]);
-    const uint32_t cap = (uint32_t)(FB_MAX_TASKS - FB_BUCKETS);
-    const uint32_t tsz = max(task, (nent + cap - 1) / cap);
-    // tasks per bucket, exclusive scan -> tstart (bucket k = 0-based index)
-    if (threadIdx.x < 32) {
-      // warp-level scan over 1024 buckets, 32 per lane
-      const int lane = threadIdx.x;
-      uint32_t loc[32];
-      uint32_t sum = 0;
-      for (int i = 0; i < 32; ++i) {
-        const int k = lane * 32 + i;
-        const uint32_t c = bcount(k);
-        loc[i] = (c + tsz - 1) / tsz;
-        sum += loc[i];
-      }
-      uint32_t incl = sum;
-      for (int d = 1; d < 32; d <<= 1) {
-        uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
-      }
-      uint32_t acc = incl - sum;
-      for (int i = 0; i < 32; ++i) {
-        tstart[lane * 32 + i] = (uint16_t)acc;
-        acc += loc[i];
-      }
-      if (lane == 31) tstart[FB_BUCKETS] = (uint16_t)acc;
-    }
-    __syncthreads();
-    const uint32_t ntasks = tstart[FB_BUCKETS];
-    // size of task j of bucket k: tsz except the bucket's last task; bin
-    // task - size * task / tsz (task - size when tsz = task): larger tasks
-    // first
-    for (int k = threadIdx.x; k < FB_BUCKETS; k += blockDim.x) {
-      const uint32_t c = bcount(k);
-      for (uint32_t t = tstart[k]; t < tstart[k + 1]; ++t) {
-        tbucket[t] = (uint16_t)k;
-        const uint32_t j = t - tstart[k];
-        const uint32_t sz = min(tsz, c - j * tsz);
-        atomicAdd(&bins[task - sz * task / tsz], 1u);
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t acc = 0;
-      for (uint32_t i = 0; i <= task; ++i) { uint32_t v = bins[i]; bins[i] = acc; acc += v; }
-    }
-    __syncthreads();
-    for (uint32_t t = threadIdx.x; t < ntasks; t += blockDim.x) {
-      const uint32_t k = tbucket[t];
-      const uint32_t c = bcount(k);
-      const uint32_t j = t - tstart[k];
-      const uint32_t sz = min(tsz, c - j * tsz);
-      order[atomicAdd(&bins[task - sz * task / tsz], 1u)] = (uint16_t)t;
-    }
-    __syncthreads();
-    for (uint32_t r = threadIdx.x; r < ntasks; r += blockDim.x) {
-      const uint32_t t = order[r];
-      const uint32_t k = tbucket[t];
-      // positions q0 .. q1 - 1 of the bucket's entries (first sort unit's
-      // c0, then the second's)
-      const uint32_t c0 = soffs[k + 1] - soffs[k];
-      const uint32_t q0 = (t - tstart[k]) * tsz;
-      const uint32_t q1 = min(q0 + tsz, bcount(k));
-      XYZZ B = XYZZ::inf();
-      for (uint32_t q = q0; q < q1; ++q) {
-        uint32_t idx, w, neg;
-        if (wide) {
-          const bool second = q >= c0;
-          const uint32_t v = second ? ents32b[soffs2[k] + (q - c0)] : ents32[soffs[k] + q];
-          idx = (v & ((1u << ulog) - 1)) + (second ? (1u << ulog) : 0u);
-          w = (v >> ulog) & 31;
-          neg = v >> 31;
-        } else {
-          const uint32_t v = ents[soffs[k] + q];
-          idx = v & 0x3ff;
-          w = (v >> 10) & 31;
-          neg = v >> 15;
-        }
-        G1Aff p = load_aff(tabl + (uint64_t)w * N + idx);
-        if (neg) p.y = -p.y;
-        B.template add_affine<M>(p.x, p.y);
-      }
-      store_xyzz(gpart + t, B);
-    }
-    __syncthreads();
-    const int k0 = threadIdx.x * FB_PER_THREAD;  // 0-based buckets k0 .. k0+7
-    XYZZ S = XYZZ::inf(), T = XYZZ::inf();
-    for (int k = k0 + FB_PER_THREAD - 1; k >= k0; --k) {
-      for (uint32_t t = tstart[k]; t < tstart[k + 1]; ++t) S.template add<M>(load_xyzz(gpart + t));
-      T.template add<M>(S);
-    }
-    store_xyzz(a.outT + (size_t)u * FB_ACC_THREADS + threadIdx.x, T);
-    store_xyzz(a.outS + (size_t)u * FB_ACC_THREADS + threadIdx.x, S);
-  }
-}
+}  // namespace zg
+#include "zg_bucket.cuh"
+namespace zg {
 
 // Where a combine launch's items go. The launch covers up to FB_MAX_SETS item
 // sets (the chunk items, then one set per wide unit size); set k holds items
@@ -1037,30 +825,31 @@ __device__ XYZZ fb_block_term(const XYZZ& P, uint32_t blk) {
   return r;
 }
 
-// Per item: P = sum_i T_i + 8 * sum_i i S_i (+ the wide block term); written
-// to part for the AMT trees.
-__global__ void __launch_bounds__(64) k_fb_combine(const XYZZ* __restrict__ T, const XYZZ* __restrict__ S,
-                                                   XYZZ* __restrict__ part, FbCombinePlan plan) {
+// Per item: P = 32 sum_a a R_a + sum_b (b + 1) C_b (+ the wide block term)
+// from its row and column sums, both by running sums; written to part for the
+// AMT trees. 128 point additions and 5 doublings per item.
+__global__ void __launch_bounds__(64) k_fb_combine(const G1Aff* __restrict__ sums, XYZZ* __restrict__ part,
+                                                   FbCombinePlan plan) {
   const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= plan.start[plan.n]) return;
   uint32_t v;
   const FbCombineMap& m = fb_plan_item(plan, u, &v);
-  const XYZZ* t = T + (size_t)u * FB_ACC_THREADS;
-  const XYZZ* s = S + (size_t)u * FB_ACC_THREADS;
-  XYZZ tot = XYZZ::inf(), run = XYZZ::inf(), wsum = XYZZ::inf();
-  for (int i = FB_ACC_THREADS - 1; i >= 1; --i) {
-    run.add(load_xyzz(s + i));
-    wsum.add(run);
-  }
-  for (int i = 0; i < FB_ACC_THREADS; ++i) tot.add(load_xyzz(t + i));
+  const G1Aff* s = sums + (size_t)u * FB_OUT;
+  XYZZ run = XYZZ::inf(), tot = XYZZ::inf();
 #pragma unroll 1
-  for (int k = 0; k < FB_PER_THREAD_LOG; ++k) wsum = wsum.dbl();  // x FB_PER_THREAD
-  tot.add(wsum);
-  const uint32_t blk = fb_item_block(m, v);
-  if (blk) {
-    run.add(load_xyzz(s));  // sum of all the item's buckets
-    tot.add(fb_block_term(run, blk));
+  for (int i = 0; i < FB_OUT; ++i) {
+    if (i == FB_GRID) {  // rows 31 .. 1 are in tot, row 0 has weight 0
+#pragma unroll 1
+      for (int k = 0; k < fb_log2(FB_GRID); ++k) tot = tot.dbl();
+      run = XYZZ::inf();
+    }
+    if (i == FB_GRID - 1) continue;
+    const G1Aff q = load_aff(s + (i < FB_GRID ? FB_GRID - 1 - i : FB_OUT + FB_GRID - 1 - i));
+    if (!aff_is_inf(q)) run.add_affine(q.x, q.y);
+    tot.add(run);
   }
+  const uint32_t blk = fb_item_block(m, v);
+  if (blk) tot.add(fb_block_term(run, blk));  // run: the sum of all the item's buckets
   XYZZ* dst = part + m.part_off + fb_part_index(m, v);
   store_xyzz(dst, tot);
   fb_fill_unused_slots(m, dst);
@@ -1080,53 +869,44 @@ __device__ __forceinline__ XYZZ shfl_xor_xyzz(const XYZZ& p, int m) {
 
 // k_fb_combine with one warp per item, for launches with few items (the
 // single MSMs of zg_ctx_msm and of slice verification: 1024 items leave
-// k_fb_combine's one thread per item on a handful of SMs). With P =
-// FB_ACC_THREADS / 32 partials per lane, lane l folds partials P l .. P l +
-// P - 1 into t_l, s_l and w_l = sum_k k S_{Pl+k}; then
-// sum_i i S_i = P sum_l l s_l + sum_l w_l, sum_l l s_l being the sum over
-// lanes l >= 1 of the suffix sums U_l = sum_{m >= l} s_m (a warp scan). About
-// three times the additions of k_fb_combine, so blob encodes keep that one.
-__global__ void __launch_bounds__(128) k_fb_combine_warp(const XYZZ* __restrict__ T, const XYZZ* __restrict__ S,
-                                                         XYZZ* __restrict__ part, FbCombinePlan plan) {
-  constexpr int P = FB_ACC_THREADS / 32;  // partials per lane
-  static_assert(P >= 1 && (P & (P - 1)) == 0, "a power of two of partials per lane");
+// k_fb_combine's one thread per item on a handful of SMs). Lane l takes row l
+// and column l; warp scans turn both into suffix sums U_l = sum_{m >= l}, and
+// sum_a a R_a = sum_{l >= 1} U_l of the rows, sum_b (b + 1) C_b = sum_l U_l of
+// the columns. 21 point operations in a row instead of 133, but about three
+// times the additions, so blob encodes keep k_fb_combine.
+__global__ void __launch_bounds__(128) k_fb_combine_warp(const G1Aff* __restrict__ sums, XYZZ* __restrict__ part,
+                                                         FbCombinePlan plan) {
   const uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (u >= plan.start[plan.n]) return;  // uniform per warp
   uint32_t v;
   const FbCombineMap& m = fb_plan_item(plan, u, &v);
-  const XYZZ* t = T + (size_t)u * FB_ACC_THREADS + P * lane;
-  const XYZZ* s = S + (size_t)u * FB_ACC_THREADS + P * lane;
-  XYZZ tl = load_xyzz(t);
-  for (int k = 1; k < P; ++k) tl.add(load_xyzz(t + k));
-  XYZZ run = XYZZ::inf(), w = XYZZ::inf();
-  for (int k = P - 1; k >= 1; --k) {
-    run.add(load_xyzz(s + k));
-    w.add(run);
+  const G1Aff* s = sums + (size_t)u * FB_OUT;
+  XYZZ U[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const G1Aff q = load_aff(s + k * FB_GRID + lane);
+    U[k] = aff_is_inf(q) ? XYZZ::inf() : XYZZ::from_affine(q);
   }
-  run.add(load_xyzz(s));
-  XYZZ U = run;
+#pragma unroll 1
   for (int d = 1; d < 32; d <<= 1) {
-    const XYZZ v = shfl_down_xyzz(U, d);
-    if (lane + d < 32) U.add(v);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const XYZZ x = shfl_down_xyzz(U[k], d);
+      if (lane + d < 32) U[k].add(x);
+    }
   }
-  XYZZ a = lane >= 1 ? U : XYZZ::inf();
-  for (int mk = 16; mk >= 1; mk >>= 1) {
-    tl.add(shfl_xor_xyzz(tl, mk));
-    w.add(shfl_xor_xyzz(w, mk));
-    a.add(shfl_xor_xyzz(a, mk));
-  }
+  XYZZ w = lane >= 1 ? U[0] : XYZZ::inf();
+#pragma unroll 1
+  for (int k = 0; k < fb_log2(FB_GRID); ++k) w = w.dbl();
+  w.add(U[1]);
+#pragma unroll 1
+  for (int mk = 16; mk >= 1; mk >>= 1) w.add(shfl_xor_xyzz(w, mk));
   if (lane == 0) {
-#pragma unroll 1
-    for (int k = 0; k < fb_log2(P); ++k) a = a.dbl();  // P sum_l l s_l
-    a.add(w);                                           // sum_i i S_i
-#pragma unroll 1
-    for (int k = 0; k < FB_PER_THREAD_LOG; ++k) a = a.dbl();  // x FB_PER_THREAD
-    tl.add(a);
     const uint32_t blk = fb_item_block(m, v);
-    if (blk) tl.add(fb_block_term(U, blk));  // U at lane 0 = sum of all the item's buckets
+    if (blk) w.add(fb_block_term(U[1], blk));  // U[1] at lane 0 = the sum of all the item's buckets
     XYZZ* dst = part + m.part_off + fb_part_index(m, v);
-    store_xyzz(dst, tl);
+    store_xyzz(dst, w);
     fb_fill_unused_slots(m, dst);
   }
 }
