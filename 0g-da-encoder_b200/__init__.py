@@ -436,8 +436,7 @@ def _read_reply(r):
         ns = L.zg_reply_num_slices(r)
         first = L.zg_reply_slice(r, 0, ctypes.byref(n))
         size = n.value
-        blob = ctypes.string_at(first, size * ns)
-        slices = [blob[i * size:(i + 1) * size] for i in range(ns)]
+        slices = [ctypes.string_at(first + i * size, size) for i in range(ns)]
         return L.zg_reply_version(r), com, root, edata, roots, slices
     finally:
         L.zg_reply_free(r)
@@ -504,7 +503,7 @@ def recover_from_da_slice(params: ZgEncoderParams, slices: dict) -> bytes:
     if rc == ZG_ERR_RECOVERY:
         raise RecoveryError(L.zg_last_error().decode())
     _check(rc)
-    return out.raw[:out_len.value]
+    return ctypes.string_at(out, out_len.value)
 
 
 class LightEncodedSlice:

@@ -34,6 +34,7 @@ struct FbAccArgs {
   int mlog = 0;                    // wide items: 2^mlog consecutive sort units share buckets
   int W = FB_WINDOWS;              // windows per table line (wd_windows(ulog) for wide items)
   uint64_t tabN = 0;               // points per window table (the param line length)
+  int group = 1;                   // items per CTA and turn
 };
 
 // One launch covers up to FB_MAX_SETS item sets (a blob's chunk items and its
@@ -70,9 +71,10 @@ constexpr int FB_GRID = 32;
 constexpr int FB_OUT = 2 * FB_GRID;
 static_assert(FB_GRID * FB_GRID == FB_BUCKETS, "buckets fill the grid");
 
-// A CTA works on up to FB_GROUP items of a set at a time: the levels of their
-// trees run together, so the short levels share their inversions.
-constexpr int FB_GROUP = 2;
+// A CTA works on up to FB_GROUP items of a set at a time (FbAccArgs::group): the
+// levels of their trees run together, so the short levels share their
+// inversions.
+constexpr int FB_GROUP = 4;
 // Per-CTA scratch, for segments of at most `cap` entries.
 struct FbScratch {
   uint8_t* base = nullptr;
@@ -90,10 +92,10 @@ struct FbScratch {
     return (off_dst() + ((size_t)cap / 2 + 16) * sizeof(uint32_t) + 255) / 256 * 256;
   }
 };
-// Largest segment per item: a 2^16-point unit's block (32 768 entries, half as
-// many again in block 0) stays in one.
-constexpr uint32_t FB_CAP_MAX = 49152;
-static_assert(FB_GROUP * (FB_CAP_MAX / 2 + 3 * FB_BUCKETS) < 65536, "slot indexes fit 16 bits");
+// Largest segment: two blocks of 2^16-point units (32 768 entries, half as many
+// again in a block 0), four chunks of 1024 points.
+constexpr uint32_t FB_CAP_MAX = 98304;
+static_assert(FB_CAP_MAX / 2 + 3 * FB_GROUP * FB_BUCKETS < 65536, "slot indexes fit 16 bits");
 
 __device__ __forceinline__ Fq ld_fq(const Fq* p) {
   const uint4* q = reinterpret_cast<const uint4*>(p);
@@ -377,14 +379,12 @@ __device__ __forceinline__ void bkt_second(Fetch fetch, Locate locate, const uin
 // merged unit and the W windows of the wide table.
 // M is the product kind of the point additions (chosen by the context's
 // tuning; identical results).
-// `group` items of a set (at most FB_GROUP, all of one launch alike) share a
-// CTA's turn.
+// A set's `group` items share a CTA's turn.
 template <class M>
 __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
-    k_fb_accum(const FbAccPlan plan, const FbScratch scratch, uint32_t* __restrict__ next, uint32_t task,
-               uint32_t group) {
+    k_fb_accum(const FbAccPlan plan, const FbScratch scratch, uint32_t* __restrict__ next, uint32_t task) {
   constexpr uint32_t T = FB_ACC_THREADS;
-  constexpr uint32_t NB = FB_GROUP * FB_BUCKETS, PER = NB / T;
+  constexpr uint32_t NB = FB_GROUP * FB_BUCKETS;
   __shared__ uint4 stg[10][T];           // the passes' staging rows
   __shared__ Fq sp[T];
   __shared__ uint16_t sstart[NB + 1];    // first slot of each bucket
@@ -400,7 +400,6 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
   uint32_t* const dst = reinterpret_cast<uint32_t*>(mem + scratch.off_dst());
   const uint32_t cap = scratch.cap;
   const uint32_t batch = fb_batch(min(max(task, (uint32_t)FB_TASK_MIN), (uint32_t)FB_TASK_MAX));
-  group = min(max(group, 1u), (uint32_t)FB_GROUP);
   uint32_t turn = blockIdx.x;
   for (;;) {
     __syncthreads();  // every thread has read the previous group number
@@ -410,13 +409,15 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     uint32_t u0 = item;
     int set = 0;
     for (; set < plan.n; ++set) {
+      const uint32_t group = (uint32_t)plan.a[set].group;
       const uint32_t groups = (plan.start[set + 1] - plan.start[set] + group - 1) / group;
       if (u0 < groups) break;
       u0 -= groups;
     }
     if (set >= plan.n) break;
-    u0 *= group;
     const FbAccArgs& a = plan.a[set];
+    const uint32_t group = (uint32_t)a.group;
+    u0 *= group;
     const uint32_t ng = min(group, plan.start[set + 1] - plan.start[set] - u0);
     const bool wide = a.ents32 != nullptr;
     // item i of the group: its bucket offsets, entries and first table point
@@ -474,7 +475,8 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     }
     __syncthreads();
     const uint32_t nent = first[ng];
-    const uint32_t k0 = tid * PER, my = k0 / FB_BUCKETS;  // this thread's buckets k0 .. are item my's
+    // this thread's buckets k0 .. k0 + per - 1 are item my's
+    const uint32_t per = (ng <= 2 ? ng : 4) * (FB_BUCKETS / T), k0 = tid * per, my = k0 / FB_BUCKETS;
     uint32_t seg = 0, st = 0, h = 0, lh = 0;
     int mode = 0;  // 0: level 1 of segment seg, 1: slots st apart, 2: grid level of half width h
     for (;;) {
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
           return p;
         };
         uint32_t cnt = 0;  // pairs | slots << 16
-        for (uint32_t k = k0; k < k0 + PER; ++k) {
+        for (uint32_t k = k0; k < k0 + per; ++k) {
           const Part p = part(k);
           cnt += ((p.n[0] >> 1) + (p.n[1] >> 1)) + ((((p.n[0] + 1) >> 1) + ((p.n[1] + 1) >> 1) + p.carry) << 16);
         }
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
         const uint32_t at = block_scan(cnt, wsum, &total);
         uint32_t p = at & 0xffffu, sl = at >> 16;
         np = total & 0xffffu;
-        for (uint32_t k = k0; k < k0 + PER; ++k) {
+        for (uint32_t k = k0; k < k0 + per; ++k) {
           const Part r = part(k);
           sstart[k] = (uint16_t)sl;
           if (r.carry) st_aff(slots + sl++, ld_aff(fin + k));
@@ -531,12 +533,12 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
             }
           }
         }
-        if (tid == T - 1) sstart[NB] = (uint16_t)sl;
+        if (tid == T - 1) sstart[k0 + per] = (uint16_t)sl;
       } else if (mode == 1) {
         uint32_t cnt = 0;
-        for (uint32_t k = k0; k < k0 + PER; ++k) cnt += ((uint32_t)sstart[k + 1] - sstart[k] + st - 1) / st >> 1;
+        for (uint32_t k = k0; k < k0 + per; ++k) cnt += ((uint32_t)sstart[k + 1] - sstart[k] + st - 1) / st >> 1;
         uint32_t p = block_scan(cnt, wsum, &np);
-        for (uint32_t k = k0; k < k0 + PER; ++k) {
+        for (uint32_t k = k0; k < k0 + per; ++k) {
           const uint32_t s0 = sstart[k], pairs = ((uint32_t)sstart[k + 1] - s0 + st - 1) / st >> 1;
           for (uint32_t i = 0; i < pairs; ++i) dst[p++] = s0 + 2 * i * st;
         }

@@ -404,6 +404,50 @@ void pinned_put(void* p, size_t bytes) {
 }
 }  // namespace
 
+// Runs fn(i) for i < n on up to 16 host threads, `grain` indexes at a time (the
+// caller's thread alone when there is one grain or threads cannot be had).
+// false if a call threw (out of memory); the other indexes still run.
+namespace {
+template <class F>
+bool host_parallel(size_t n, size_t grain, F fn) {
+  std::atomic<size_t> next{0};
+  std::atomic<bool> ok{true};
+  auto work = [&] {
+    for (size_t b; (b = next.fetch_add(grain)) < n;)
+      for (size_t i = b; i < std::min(n, b + grain); ++i) {
+        try {
+          fn(i);
+        } catch (...) {
+          ok = false;
+        }
+      }
+  };
+  const size_t blocks = (n + grain - 1) / grain;
+  const size_t want = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), blocks});
+  std::vector<std::thread> more;
+  try {
+    more.reserve(want);
+    for (size_t t = 1; t < want; ++t) more.emplace_back(work);
+  } catch (...) {
+  }
+  work();
+  for (std::thread& t : more) t.join();
+  return ok;
+}
+// memcpy, by several threads from 4 MiB on: one thread moves some 8 GB/s
+// between pageable and pinned memory, a blob's rows are 50 MB
+void host_copy(void* dst, const void* src, size_t n) {
+  constexpr size_t kPart = 1 << 20;
+  if (n < 4 * kPart) {
+    memcpy(dst, src, n);
+    return;
+  }
+  host_parallel((n + kPart - 1) / kPart, 1, [&](size_t i) {
+    memcpy((uint8_t*)dst + i * kPart, (const uint8_t*)src + i * kPart, std::min(kPart, n - i * kPart));
+  });
+}
+}  // namespace
+
 struct zg_reply {
   uint32_t version = 0;
   uint8_t commitment[64];
@@ -490,12 +534,13 @@ uint32_t blob_items(const zg_ctx* c) {
   return u;
 }
 
-// k_fb_accum's segment size: the entries of a group of a context's largest
-// items, with half as many again for a wide unit's block 0
+// k_fb_accum's segment size: the entries of FB_GROUP of a context's largest
+// items, a wide unit's block 0 counted with half as many again, within
+// FB_CAP_MAX
 uint32_t fb_segment(const zg_ctx* c) {
   uint32_t n = (uint32_t)(FB_WINDOWS * c->C);
   for (const zg_ctx::WdClass& k : c->wd) n = std::max(n, ((uint32_t)wd_windows(k.ulog) * 1536u) << k.mlog);
-  return (uint32_t)FB_GROUP * std::min(n, FB_CAP_MAX);
+  return std::min((uint32_t)FB_GROUP * n, FB_CAP_MAX);
 }
 
 // device bytes of a lane of `cap` blob slots (the request pipeline's
@@ -744,20 +789,32 @@ int check_launch() {
   return 0;
 }
 
-// Leaves, then one launch per level down to MERKLE_TOP_MAX, then the levels
-// above in one k_merkle_top launch (off[d] = 96 (2^d - 1), the layout it
-// assumes).
-int merkle_levels(const uint8_t* items, size_t n_items, uint8_t* tree, const std::vector<uint64_t>& off,
-                  int depth, cudaStream_t s) {
-  const unsigned T = 128;
-  size_t leaves = n_items / 8;
-  k_merkle_leaves<<<nblk(leaves, T), T, 0, s>>>(items, tree + off[depth], (uint32_t)leaves);
+// The tree of n_items / 8 = 3 * 2^depth leaves (level d at 96 (2^d - 1) of
+// `tree`): one launch per level while it fills the GPU (a CTA that goes on to
+// the levels above its nodes leaves its SM with half of its warps, then a
+// quarter: leaves and two levels in one launch 319 us, in three 271), from
+// MERKLE_WIDE_MIN on three levels per launch, and the levels below
+// MERKLE_TOP_MAX in one k_merkle_top launch. launch(kind, d, up) is called
+// for each: 0 leaves, 1 parents with `up` levels above them, 2 top.
+constexpr int MERKLE_WIDE_MIN = 15;
+template <class Launch>
+void merkle_plan(int depth, Launch launch) {
   const int top = std::min(depth, MERKLE_TOP_MAX);
-  for (int d = depth - 1; d >= top; --d) {
-    size_t cnt = (size_t)3 << d;
-    k_merkle_parents<<<nblk(cnt, T), T, 0, s>>>(tree + off[d + 1], tree + off[d], (uint32_t)cnt);
+  launch(0, depth, 0);
+  for (int d = depth, n; d > top; d -= n) {
+    n = d > MERKLE_WIDE_MIN ? 1 : std::min(3, d - top);
+    launch(1, d, n - 1);
   }
-  if (top > 0) k_merkle_top<<<3, std::max(1, 1 << (top - 1)), 0, s>>>(tree, top);
+  if (top > 0) launch(2, top, 0);
+}
+int merkle_levels(const uint8_t* items, size_t n_items, uint8_t* tree, int depth, cudaStream_t s) {
+  const unsigned T = MERKLE_THREADS;
+  const size_t leaves = n_items / 8;
+  merkle_plan(depth, [&](int kind, int d, int up) {
+    if (kind == 0) k_merkle_leaves<<<nblk(leaves, T), T, 0, s>>>(items, tree, depth, (uint32_t)leaves);
+    else if (kind == 1) k_merkle_parents<<<(unsigned)(((size_t)3 << d) / (2 * T)), T, 0, s>>>(tree, d, up);
+    else k_merkle_top<<<3, std::max(1, 1 << (d - 1)), 0, s>>>(tree, d);
+  });
   return check_launch();
 }
 
@@ -793,8 +850,8 @@ BlobBufs ctx_bufs(zg_ctx* c) {
 // (and its counter reset) and the combine (the 8-bit path: chunks + combine
 // per blob).
 uint64_t launches_per_encode(const zg_ctx* c, int nb = 1) {
-  const int top = std::min(c->tree_depth, MERKLE_TOP_MAX);
-  const uint64_t merkle = 1 + (uint64_t)(c->tree_depth - top) + (top > 0 ? 1 : 0);
+  uint64_t merkle = 0;
+  merkle_plan(c->tree_depth, [&](int, int, int) { ++merkle; });
   uint64_t sorts = 0;  // the wide classes in use that run their own digit sort
   for (int k = 0; k < c->wd_on; ++k) sorts += c->wd[k].sort_of == k ? 1 : 0;
   const uint64_t per = 3 + merkle + 1 + (c->fb ? 1 + sorts : 2) + 1 + 1 + 1;
@@ -902,16 +959,42 @@ __global__ void k_fill_payload(uint8_t* p, uint64_t n, uint64_t seed) {
   }
 }
 
+// Items per CTA and turn of each set: the number g <= FB_GROUP that fits the
+// scratch (four fifths of it by the items' usual entries: a wide unit's block
+// 0 holds up to half as many again, and a group beyond the scratch would run
+// in two segments) and makes rounds x (g entries + FB_TURN_ENTS) smallest,
+// FB_TURN_ENTS being the cost of a turn's chain of inversions (16 of 35 us)
+// in entries at four CTAs per SM. Returns the turns in all.
+constexpr uint32_t FB_TURN_ENTS = 12000;
+uint32_t fb_choose_groups(FbAccPlan& p, uint32_t ctas, uint32_t cap) {
+  uint32_t turns = 0;
+  const uint32_t units = p.start[p.n];
+  for (int k = 0; k < p.n; ++k) {
+    FbAccArgs& a = p.a[k];
+    const uint32_t ents = a.ents32 ? ((uint32_t)a.W * FB_BUCKETS) << a.mlog : (uint32_t)FB_WINDOWS << a.lc;
+    uint64_t best = UINT64_MAX;
+    for (uint32_t g = 1; g <= (uint32_t)FB_GROUP && (g == 1 || (uint64_t)g * ents * 5 <= (uint64_t)cap * 4); ++g) {
+      const uint64_t rounds = (units + g * ctas - 1) / (g * ctas);
+      const uint64_t cost = rounds * ((uint64_t)g * (ents + 2 * FB_BUCKETS) + FB_TURN_ENTS);
+      if (cost < best) {
+        best = cost;
+        a.group = (int)g;
+      }
+    }
+    turns += (p.start[k + 1] - p.start[k] + a.group - 1) / a.group;
+  }
+  return turns;
+}
+
 // k_fb_accum over the item sets of `p` with product kind `kind`, on a lane's
 // counter and task scratch
-void launch_fb_accum(const zg_ctx* c, const Lane& ln, uint32_t kind, const FbAccPlan& p, cudaStream_t s) {
-  const uint32_t units = p.start[p.n];
-  // two items per CTA and turn once every resident CTA has that many
-  const uint32_t group = units >= 2 * c->fb_ctas[kind] ? FB_GROUP : 1;
-  const unsigned grid = std::min<unsigned>(c->fb_ctas[kind], (units + group - 1) / group);
+void launch_fb_accum(const zg_ctx* c, const Lane& ln, uint32_t kind, const FbAccPlan& plan, cudaStream_t s) {
+  FbAccPlan p = plan;
+  const uint32_t turns = fb_choose_groups(p, c->fb_ctas[kind], ln.fb_scratch.cap);
+  const unsigned grid = std::min<unsigned>(c->fb_ctas[kind], turns);
   cudaMemsetAsync(ln.fb_next, 0, sizeof(uint32_t), s);
   auto go = [&](auto kernel) {
-    kernel<<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_scratch, ln.fb_next, c->msm_task, group);
+    kernel<<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_scratch, ln.fb_next, c->msm_task);
   };
   switch (kind) {
     case ZG_MSM_PRODUCT_IMAD: go(k_fb_accum<MulImad>); break;
@@ -973,6 +1056,26 @@ void launch_fb_combine(const Lane& ln, const FbCombinePlan& p, cudaStream_t s) {
   if (units >= 16384) k_fb_combine<<<nblk(units, 64), 64, 0, s>>>(ln.fb_out, ln.part, p);
   else k_fb_combine_warp<<<nblk((size_t)units * 32, 128), 128, 0, s>>>(ln.fb_out, ln.part, p);
 }
+
+// out[y] = sum of the n points at in + y stride, y < sets: one CTA per 512
+// points, then one over their results (tmp: sets * 64 points); returns the
+// kernels launched
+int launch_sum_points(const XYZZ* in, uint32_t n, uint64_t stride, uint32_t sets, XYZZ* tmp, XYZZ* out,
+                      cudaStream_t s) {
+  const uint32_t ctas = std::min(64u, (n + 511) / 512);
+  if (ctas <= 1) {
+    k_sum_points<<<dim3(1, sets), SUM_THREADS, 0, s>>>(in, n, stride, out);
+    return 1;
+  }
+  k_sum_points<<<dim3(ctas, sets), SUM_THREADS, 0, s>>>(in, n, stride, tmp);
+  k_sum_points<<<dim3(1, sets), SUM_THREADS, 0, s>>>(tmp, ctas, ctas, out);
+  return 2;
+}
+
+// Splits of a single MSM of 2^logn points by k_fs_accum (0: k_fb_accum): 2^12
+// points each, so that a thread sums some 6 entries.
+constexpr int FS_MAX_LOG = 15;
+uint32_t fs_splits(int logn) { return logn > FS_MAX_LOG ? 0 : 1u << std::max(0, logn - 12); }
 
 // k_wd_sort / k_wd_tables for a class's unit size
 void launch_wd_sort(int ulog, const uint8_t* enc, uint32_t* offs, uint32_t* ents, int lr, int lc, size_t N,
@@ -1039,7 +1142,7 @@ int encode_launches(zg_ctx* c, const Lane& ln, const BlobBufs* b, int nb, const 
   mark(1);
   // Merkle tree over the encoded data and the file root
   for (int i = 0; i < nb; ++i) {
-    if ((rc = merkle_levels(b[i].enc, 3 * N, b[i].tree, c->tree_off, c->tree_depth, s))) return rc;
+    if ((rc = merkle_levels(b[i].enc, 3 * N, b[i].tree, c->tree_depth, s))) return rc;
     k_file_root<<<1, 32, 0, s>>>(b[i].tree + c->tree_off[0], b[i].file_root);
   }
   mark(2);
@@ -1085,7 +1188,7 @@ int encode_launches(zg_ctx* c, const Lane& ln, const BlobBufs* b, int nb, const 
   for (int i = 0; i < nb; ++i) {
     XYZZ* part = ln.part + (size_t)i * 3 * c->L * R;
     XYZZ* nodes = ln.nodes + (size_t)i * nn;
-    k_amt_tree<<<dim3((unsigned)c->L, 3), 256, 0, s>>>(part, nodes, lr, c->L);
+    k_amt_tree<<<dim3((unsigned)c->L, 3), std::min(AMT_THREADS, std::max(32, 2 << c->lr)), 0, s>>>(part, nodes, lr, c->L);
     k_serialize_nodes<<<nblk(nn, 128), 128, 0, s>>>(nodes, b[i].amt, nn);
   }
   mark(4);
@@ -1501,7 +1604,7 @@ int issue_unit(Engine* e, Unit* u) {
     cudaPointerAttributes pa;
     if (lens[i] && (cudaPointerGetAttributes(&pa, src[i]) != cudaSuccess || pa.type != cudaMemoryTypeHost)) {
       cudaGetLastError();
-      memcpy(u->h_stage[i], src[i], lens[i]);
+      host_copy(u->h_stage[i], src[i], lens[i]);
       src[i] = u->h_stage[i];
     }
     const uint64_t len64 = lens[i];
@@ -1928,20 +2031,28 @@ struct Coeffs {
   uint64_t s = 0;
   bool os = false;
   bool failed = false;  // the OS generator did not answer
+  uint32_t pool[4096];  // drawn from the OS, not yet handed out: pool[at ..]
+  size_t at = 4096;
   void next(uint32_t w[4]) {
     if (os) {
-      uint8_t* p = reinterpret_cast<uint8_t*>(w);
-      size_t got = 0;
-      while (got < 16) {
-        const ssize_t k = getrandom(p + got, 16 - got, 0);
-        if (k < 0) {
-          if (errno == EINTR) continue;
-          failed = true;
-          memset(w, 0, 16);
-          return;
+      if (at + 4 > 4096) {  // a system call per 1024 coefficients
+        uint8_t* p = reinterpret_cast<uint8_t*>(pool);
+        size_t got = 0;
+        while (got < sizeof(pool)) {
+          const ssize_t k = getrandom(p + got, sizeof(pool) - got, 0);
+          if (k < 0) {
+            if (errno == EINTR) continue;
+            failed = true;
+            memset(w, 0, 16);
+            return;
+          }
+          got += (size_t)k;
         }
-        got += (size_t)k;
+        at = 0;
       }
+      memcpy(w, pool + at, 16);
+      memset(pool + at, 0, 16);
+      at += 4;
       return;
     }
     for (int k = 0; k < 2; ++k) {
@@ -1951,11 +2062,32 @@ struct Coeffs {
     }
   }
 };
-Fr fr_of_words(const uint32_t w[4]) {
-  Fr x = Fr::zero();
-  for (int i = 0; i < 4; ++i) x.v[i] = w[i];
-  return Fr::from_canonical(x);
+// the coefficient k1 + lambda k2 of the words w (k1 = w[0..1], k2 = w[2..3];
+// lambda the eigenvalue of the curve endomorphism, see zg_verify.cuh)
+Fr fr_of_coeff(const uint32_t w[4]) {
+  Fr lambda;  // Montgomery form
+  const uint32_t l[8] = {0x4a0329b3u, 0x93e7cedeu, 0x7a96c167u, 0x7d4fdca7u,
+                         0xb19a750au, 0x8be4ba08u, 0xa5661c25u, 0x1cbd5653u};
+  for (int i = 0; i < 8; ++i) lambda.v[i] = l[i];
+  Fr a = Fr::zero(), b = Fr::zero();
+  a.v[0] = w[0]; a.v[1] = w[1];
+  b.v[0] = w[2]; b.v[1] = w[3];
+  return Fr::from_canonical(a) + Fr::from_canonical(b) * lambda;
 }
+// sums of the two 64-bit halves of coefficients, 96 bits each
+struct CoeffSum {
+  unsigned __int128 k[2] = {0, 0};
+  void add(const uint32_t w[4]) {
+    for (int h = 0; h < 2; ++h) k[h] += (uint64_t)w[2 * h + 1] << 32 | w[2 * h];
+  }
+  void add(const CoeffSum& o) {
+    for (int h = 0; h < 2; ++h) k[h] += o.k[h];
+  }
+  void words(std::vector<uint32_t>& out) const {
+    for (int h = 0; h < 2; ++h)
+      for (int i = 0; i < 3; ++i) out.push_back((uint32_t)(k[h] >> (32 * i)));
+  }
+};
 
 // device scratch of one zg_verify_slices call
 struct VerifyRun {
@@ -1967,7 +2099,7 @@ struct VerifyRun {
   uint64_t stride = 0;
   std::vector<uint32_t> dpos;   // slice index -> position in d_slices
   uint8_t* d_scal = nullptr;    // [3][N] canonical scalars of the MSM checks
-  Coeffs rng{0};
+  Coeffs rng;
   std::vector<void*> owned;
   template <class T>
   T* dev(size_t n) {
@@ -1985,31 +2117,37 @@ struct VerifyRun {
 uint32_t slice_coset(const zg_ctx* c, const PSlice& p) { return (uint32_t)(p.amt_index / c->R); }
 uint32_t slice_bi(const zg_ctx* c, const PSlice& p) { return host_brev((uint32_t)(p.row_index), c->lr); }
 
-// MSM over every coset's basis line with the scalars in d_scal (cosets with
-// present[c]); out[c] on the device
+// MSMs over the basis lines of the cosets with present[c], scalars in d_scal,
+// in one accumulation; out[k] (device, three points) of the k-th present coset
 int verify_msms(VerifyRun& v, const bool present[3], XYZZ* out) {
   zg_ctx* c = v.c;
   const uint32_t R = (uint32_t)c->R;
+  XYZZ* tmp = v.dev<XYZZ>(3 * 64);
+  if (!tmp) return fail(ZG_ERR_CUDA, "verify: device allocation failed");
+  FbAccPlan acc;
+  FbCombinePlan comb;
   for (int cs = 0; cs < 3; ++cs) {
     if (!present[cs]) continue;
-    k_fb_sort<<<dim3(R, 1), 256, fb_sort_smem_bytes(c->lc), v.s>>>(v.d_scal + (size_t)cs * c->N * 32, c->lane.fb_offs,
-                                                                   c->lane.fb_ents, c->lr, c->lc, 0, 0);
-    FbAccArgs fa;
+    const uint32_t k = (uint32_t)acc.n;
+    FbAccArgs& fa = acc.a[k];
+    uint32_t* offs = c->lane.fb_offs + (size_t)k * R * (FB_BUCKETS + 1);
+    uint16_t* ents = c->lane.fb_ents + (size_t)k * R * FB_WINDOWS * c->C;
+    k_fb_sort<<<dim3(R, 1), 256, fb_sort_smem_bytes(c->lc), v.s>>>(v.d_scal + (size_t)cs * c->N * 32, offs, ents, c->lr,
+                                                                   c->lc, 0, 0);
     fa.tab = c->line_ptr(cs, c->lr);
-    fa.offs = c->lane.fb_offs;
-    fa.ents = c->lane.fb_ents;
-    fa.out = c->lane.fb_out;
-    fa.ents32 = nullptr;
+    fa.offs = offs;
+    fa.ents = ents;
+    fa.out = c->lane.fb_out + (size_t)k * R * FB_OUT;
     fa.lr = c->lr;
     fa.lc = c->lc;
-    fa.lines = 1;
-    fa.l0 = 0;
-    fa.Ltot = 1;
     fa.tabN = c->N;
-    launch_fb_accum(c, c->lane, c->msm_product, single_acc_plan(fa, R), v.s);
-    launch_fb_combine(c->lane, single_fb_plan(c->lr), v.s);
-    k_sum_points<<<1, 256, 0, v.s>>>(c->lane.part, R, out + cs);
+    comb.m[k] = FbCombineMap{c->lr, 1, 0, 1, 0, 0, 0, (uint64_t)k * R};
+    acc.start[++acc.n] = (k + 1) * R;
+    comb.start[++comb.n] = (k + 1) * R;
   }
+  launch_fb_accum(c, c->lane, c->msm_product, acc, v.s);
+  launch_fb_combine(c->lane, comb, v.s);
+  launch_sum_points(c->lane.part, R, R, (uint32_t)acc.n, tmp, out, v.s);
   return check_launch();
 }
 
@@ -2041,16 +2179,16 @@ int amt_batch(VerifyRun& v, const std::vector<uint32_t>& ids, bool* ok) {
   bool present[3] = {false, false, false};
   std::vector<uint32_t> h_pos(n), h_cos(n), h_bi(n);
   std::vector<Fr> h_alpha(n);
-  Fr asum[3] = {Fr::zero(), Fr::zero(), Fr::zero()}, gsum[3] = {Fr::zero(), Fr::zero(), Fr::zero()};
+  CoeffSum asum, gsum[3];
   for (size_t j = 0; j < n; ++j) {
     const PSlice& p = sl[ids[j]];
     h_pos[j] = v.dpos[ids[j]];
     h_cos[j] = slice_coset(c, p);
     h_bi[j] = slice_bi(c, p);
-    h_alpha[j] = fr_of_words(&alpha_w[4 * j]);
+    h_alpha[j] = fr_of_coeff(&alpha_w[4 * j]);
     present[h_cos[j]] = true;
-    asum[h_cos[j]] = asum[h_cos[j]] + h_alpha[j];
-    gsum[h_cos[j]] = gsum[h_cos[j]] + fr_of_words(&gamma_w[4 * j]);
+    asum.add(&alpha_w[4 * j]);
+    gsum[h_cos[j]].add(&gamma_w[4 * j]);
   }
   uint32_t* d_pos = v.dev<uint32_t>(n);
   uint32_t* d_cos = v.dev<uint32_t>(n);
@@ -2069,7 +2207,8 @@ int amt_batch(VerifyRun& v, const std::vector<uint32_t>& ids, bool* ok) {
   if (!d_msm) return fail(ZG_ERR_CUDA, "verify: device allocation failed");
   int rc = verify_msms(v, present, d_msm);
   if (rc) return rc;
-  // weighted G1 terms: [L: comm (beta), high (gamma)] [G: quot (beta), by group] [D: comm (alpha)]
+  // weighted G1 terms: [L: comm (beta), high (gamma)] [G: quot (beta), by group];
+  // [D: per slice alpha sum_d comm_d]
   std::vector<uint32_t> gkey(n * LR);
   std::vector<uint32_t> gcount((size_t)3 * per, 0);
   for (size_t j = 0; j < n; ++j)
@@ -2085,7 +2224,7 @@ int amt_batch(VerifyRun& v, const std::vector<uint32_t>& ids, bool* ok) {
       goff.push_back(goff.back() + gcount[k]);
     }
   const uint32_t ng = (uint32_t)goff.size() - 1;
-  const size_t nL = n * (LR + 1), nG = n * LR, nD = n * LR, nt = nL + nG + nD;
+  const size_t nL = n * (LR + 1), nG = n * LR, nt = nL + nG;
   std::vector<G1Aff> tp(nt);
   std::vector<uint8_t> tinf(nt);
   std::vector<uint32_t> tsc(4 * nt);
@@ -2100,49 +2239,53 @@ int amt_batch(VerifyRun& v, const std::vector<uint32_t>& ids, bool* ok) {
     for (int d = 0; d < LR; ++d) {
       put(j * (LR + 1) + d, p.comm[d], &beta_w[4 * (j * LR + d)]);
       put(nL + fill[gid[gkey[j * LR + d]]]++, p.quot[d], &beta_w[4 * (j * LR + d)]);
-      put(nL + nG + j * LR + d, p.comm[d], &alpha_w[4 * j]);
     }
     put(j * (LR + 1) + LR, p.high, &gamma_w[4 * j]);
   }
   G1Aff* d_tp = v.dev<G1Aff>(nt);
   uint8_t* d_tinf = v.dev<uint8_t>(nt);
   uint32_t* d_tsc = v.dev<uint32_t>(4 * nt);
-  XYZZ* d_terms = v.dev<XYZZ>(nt);
+  XYZZ* d_terms = v.dev<XYZZ>(nt + n);
+  uint32_t* d_aw = v.dev<uint32_t>(4 * n);
+  XYZZ* d_sum = v.dev<XYZZ>(64);
   uint32_t* d_goff = v.dev<uint32_t>(goff.size());
   // pairing inputs: [0] L, [1..ng] G_g, then H_c per present coset; extra: D sum, A, H scalars
   const uint32_t npair = 1 + ng + (present[0] + present[1] + present[2]);
   XYZZ* d_pin = v.dev<XYZZ>(npair + 2);  // + D sum, A = (sum alpha) commitment
-  if (!d_tp || !d_tinf || !d_tsc || !d_terms || !d_goff || !d_pin) return fail(ZG_ERR_CUDA, "verify: allocation");
+  if (!d_tp || !d_tinf || !d_tsc || !d_terms || !d_aw || !d_sum || !d_goff || !d_pin) return fail(ZG_ERR_CUDA, "verify: allocation");
   ZG_CK(cudaMemcpyAsync(d_tp, tp.data(), nt * sizeof(G1Aff), cudaMemcpyHostToDevice, v.s));
   ZG_CK(cudaMemcpyAsync(d_tinf, tinf.data(), nt, cudaMemcpyHostToDevice, v.s));
   ZG_CK(cudaMemcpyAsync(d_tsc, tsc.data(), 16 * nt, cudaMemcpyHostToDevice, v.s));
   ZG_CK(cudaMemcpyAsync(d_goff, goff.data(), 4 * goff.size(), cudaMemcpyHostToDevice, v.s));
-  k_g1_mul_words<<<nblk(nt, 128), 128, 0, v.s>>>(d_tp, d_tinf, d_tsc, 4, d_terms, (uint32_t)nt);
-  k_sum_points<<<1, 256, 0, v.s>>>(d_terms, (uint32_t)nL, d_pin);
-  k_seg_sum<<<nblk(ng, 128), 128, 0, v.s>>>(d_terms + nL, d_goff, d_pin + 1, ng);
-  k_sum_points<<<1, 256, 0, v.s>>>(d_terms + nL + nG, (uint32_t)nD, d_pin + npair);
-  // full-size multiples of the commitment: H_c = (sum gamma over c) C, A = (sum alpha) C
+  ZG_CK(cudaMemcpyAsync(d_aw, alpha_w.data(), 16 * n, cudaMemcpyHostToDevice, v.s));
+  k_g1_mul_glv<<<nblk(nt, 128), 128, 0, v.s>>>(d_tp, d_tinf, d_tsc, d_terms, (uint32_t)nt);
+  launch_sum_points(d_terms, (uint32_t)nL, 0, 1, d_sum, d_pin, v.s);
+  k_seg_sum<<<nblk((size_t)ng * 32, 128), 128, 0, v.s>>>(d_terms + nL, d_goff, d_pin + 1, ng);
+  k_g1_mul_sum<<<nblk(4 * n, 128), 128, 0, v.s>>>(d_tp, d_tinf, (uint32_t)LR, (uint32_t)LR + 1, d_aw, 2, d_terms + nt,
+                                                  (uint32_t)n);
+  launch_sum_points(d_terms + nt, (uint32_t)n, 0, 1, d_sum, d_pin + npair, v.s);
+  // multiples of the commitment by coefficient sums: H_c = (sum gamma over c) C, A = (sum alpha) C
   std::vector<uint32_t> big;
   std::vector<G1Aff> bigp;
-  Fr atot = asum[0] + asum[1] + asum[2];
   for (int cs = 0; cs < 4; ++cs) {
     if (cs < 3 && !present[cs]) continue;
-    const Fr k = (cs < 3 ? gsum[cs] : atot).to_canonical();
-    big.insert(big.end(), k.v, k.v + 8);
+    (cs < 3 ? gsum[cs] : asum).words(big);
     bigp.push_back(v.auth.p);
   }
   const uint32_t nb = (uint32_t)bigp.size();
   G1Aff* d_bp = v.dev<G1Aff>(nb);
   uint8_t* d_binf = v.dev<uint8_t>(nb);
-  uint32_t* d_bsc = v.dev<uint32_t>(8 * nb);
-  if (!d_bp || !d_binf || !d_bsc) return fail(ZG_ERR_CUDA, "verify: allocation");
+  uint32_t* d_bsc = v.dev<uint32_t>(6 * nb);
+  XYZZ* d_big = v.dev<XYZZ>(nb);
+  if (!d_bp || !d_binf || !d_bsc || !d_big) return fail(ZG_ERR_CUDA, "verify: allocation");
   std::vector<uint8_t> binf(nb, v.auth.inf);
   ZG_CK(cudaMemcpyAsync(d_bp, bigp.data(), nb * sizeof(G1Aff), cudaMemcpyHostToDevice, v.s));
   ZG_CK(cudaMemcpyAsync(d_binf, binf.data(), nb, cudaMemcpyHostToDevice, v.s));
-  ZG_CK(cudaMemcpyAsync(d_bsc, big.data(), 32 * nb, cudaMemcpyHostToDevice, v.s));
-  // H_c land after the groups, A after the D sum
-  k_g1_mul_words<<<1, 128, 0, v.s>>>(d_bp, d_binf, d_bsc, 8, d_pin + 1 + ng, nb - 1);
-  k_g1_mul_words<<<1, 128, 0, v.s>>>(d_bp + nb - 1, d_binf + nb - 1, d_bsc + 8 * (nb - 1), 8, d_pin + npair + 1, 1);
+  ZG_CK(cudaMemcpyAsync(d_bsc, big.data(), 24 * nb, cudaMemcpyHostToDevice, v.s));
+  // H_c go after the groups, A after the D sum
+  k_g1_mul_sum<<<1, 128, 0, v.s>>>(d_bp, d_binf, 1, 1, d_bsc, 3, d_big, nb);
+  ZG_CK(cudaMemcpyAsync(d_pin + 1 + ng, d_big, (nb - 1) * sizeof(XYZZ), cudaMemcpyDeviceToDevice, v.s));
+  ZG_CK(cudaMemcpyAsync(d_pin + npair + 1, d_big + nb - 1, sizeof(XYZZ), cudaMemcpyDeviceToDevice, v.s));
   // MSM check on the host
   XYZZ hm[3], hd[2];
   ZG_CK(cudaMemcpyAsync(hm, d_msm, sizeof(hm), cudaMemcpyDeviceToHost, v.s));
@@ -2161,20 +2304,19 @@ int amt_batch(VerifyRun& v, const std::vector<uint32_t>& ids, bool* ok) {
   G1Aff* d_pa = v.dev<G1Aff>(npair);
   uint8_t* d_pinf = v.dev<uint8_t>(npair);
   Fq12* d_f = v.dev<Fq12>(npair);
-  Fq12* d_part = v.dev<Fq12>(128);
+  Fq12* d_part = v.dev<Fq12>(FQ12_PARTS);
   if (!d_q || !d_neg || !d_pa || !d_pinf || !d_f || !d_part) return fail(ZG_ERR_CUDA, "verify: allocation");
   ZG_CK(cudaMemcpyAsync(d_q, q.data(), npair * sizeof(G2Aff), cudaMemcpyHostToDevice, v.s));
   ZG_CK(cudaMemcpyAsync(d_neg, neg.data(), npair, cudaMemcpyHostToDevice, v.s));
   k_pairing_inputs<<<nblk(npair, 128), 128, 0, v.s>>>(d_pin, d_neg, d_pa, d_pinf, npair);
-  k_miller<<<nblk(npair, 64), 64, 0, v.s>>>(d_pa, d_pinf, d_q, d_f, npair);
-  k_fq12_partial<<<1, 128, 0, v.s>>>(d_f, npair, d_part);
-  std::vector<Fq12> part(128);
-  ZG_CK(cudaMemcpyAsync(part.data(), d_part, 128 * sizeof(Fq12), cudaMemcpyDeviceToHost, v.s));
+  k_miller<<<nblk(2 * (size_t)npair, 64), 64, 0, v.s>>>(d_pa, d_pinf, d_q, d_f, npair);
+  k_fq12_partial<<<FQ12_PARTS, 32, 0, v.s>>>(d_f, npair, d_part);
+  std::vector<Fq12> part(FQ12_PARTS);
+  ZG_CK(cudaMemcpyAsync(part.data(), d_part, FQ12_PARTS * sizeof(Fq12), cudaMemcpyDeviceToHost, v.s));
   if ((rc = check_launch())) return rc;
   ZG_CK(cudaStreamSynchronize(v.s));
   XYZZ left = XYZZ::inf();
-  for (int cs = 0; cs < 3; ++cs)
-    if (present[cs]) left.add(hm[cs]);
+  for (int k = 0; k < present[0] + present[1] + present[2]; ++k) left.add(hm[k]);
   left.add(hd[0]);
   const bool ok_msm = xyzz_eq(left, hd[1]);
   Fq12 f = Fq12::one();
@@ -2229,7 +2371,7 @@ int amt_single(VerifyRun& v, uint32_t id, int* sub, int64_t* kzg_d) {
   int rc = verify_msms(v, present, d_msm);
   if (rc) return rc;
   XYZZ m;
-  ZG_CK(cudaMemcpyAsync(&m, d_msm + cs, sizeof(XYZZ), cudaMemcpyDeviceToHost, v.s));
+  ZG_CK(cudaMemcpyAsync(&m, d_msm, sizeof(XYZZ), cudaMemcpyDeviceToHost, v.s));
   ZG_CK(cudaStreamSynchronize(v.s));
   for (int d = 0; d < LR; ++d)
     if (!p.comm[d].inf) m.add_affine(p.comm[d].p.x, p.comm[d].p.y);
@@ -2414,7 +2556,7 @@ int zg_encode(zg_ctx* c, const uint8_t* data, size_t len, int require_data, zg_r
   cudaPointerAttributes pa;
   if (len && (cudaPointerGetAttributes(&pa, data) != cudaSuccess || pa.type != cudaMemoryTypeHost)) {
     cudaGetLastError();
-    memcpy(c->h_in, data, len);
+    host_copy(c->h_in, data, len);
     src = c->h_in;
   }
   if (len && cudaMemcpyAsync(c->raw, src, len, cudaMemcpyHostToDevice, s) != cudaSuccess)
@@ -2660,10 +2802,17 @@ int zg_verify_slices(zg_ctx* c, const uint8_t* const* slices, const size_t* lens
   // amt/slice.rs:53-103; verify_amt_proof's length checks, verify_params.rs:147-160)
   std::vector<uint32_t> batch;
   size_t maxlen = 0;
+  // the deserialization on the host's threads (22 on-curve checks and 1024
+  // range checks per production slice)
+  std::vector<uint8_t> parsed(n, 0);
+  if (!host_parallel(n, 8, [&](size_t i) {
+        parsed[i] = auth_ok && slices[i] && parse_slice(slices[i], lens[i], &sl[i]);
+      }))
+    return fail(ZG_ERR_INTERNAL, "verify: out of host memory");
   for (size_t i = 0; i < n; ++i) {
     int64_t* d = &det[4 * i];
     PSlice& p = sl[i];
-    if (!auth_ok || !slices[i] || !parse_slice(slices[i], lens[i], &p)) { codes[i] = 30; continue; }
+    if (!parsed[i]) { codes[i] = 30; continue; }
     const uint64_t coset = p.amt_index / R, local = p.amt_index % R;
     if (p.index != p.amt_index) { codes[i] = 1; d[1] = (int64_t)p.index; d[2] = (int64_t)p.amt_index; }
     else if (p.index != p.leaf_index) { codes[i] = 2; d[1] = (int64_t)p.index; d[2] = (int64_t)p.leaf_index; }
@@ -2693,9 +2842,9 @@ int zg_verify_slices(zg_ctx* c, const uint8_t* const* slices, const size_t* lens
     for (size_t j = 0; j < nb; ++j) {
       const uint32_t i = batch[j];
       v.dpos[i] = (uint32_t)j;
-      memcpy(stage + j * v.stride, slices[i], lens[i]);
       nproof[j] = (uint32_t)sl[i].nmerkle;
     }
+    host_parallel(nb, 8, [&](size_t j) { memcpy(stage + j * v.stride, slices[batch[j]], lens[batch[j]]); });
     v.d_slices = v.dev<uint8_t>(nb * v.stride);
     v.d_scal = v.dev<uint8_t>(3 * c->N * 32);
     uint32_t* d_np = v.dev<uint32_t>(nb);
@@ -3068,13 +3217,16 @@ int zg_recover(zg_ctx* c, const uint64_t* row_ids, const uint8_t* const* rows, c
   std::vector<uint32_t> ids;
   std::vector<uint8_t> known(M, 0);
   size_t k = 0;
+  std::vector<const uint8_t*> from;
   for (auto& kv : valid) {
-    memcpy(c->h_rec + k * 32 * C, kv.second, 32 * C);
+    from.push_back(kv.second);
     ids.push_back((uint32_t)kv.first);
     const uint32_t cs = (uint32_t)(kv.first >> lr), r = (uint32_t)(kv.first & (R - 1));
     known[4 * r + (cs == 1 ? 2 : (cs == 2 ? 1 : cs))] = 1;
     ++k;
   }
+  host_parallel(k, std::max<size_t>(1, (1 << 18) / (32 * C)),
+                [&](size_t i) { memcpy(c->h_rec + i * 32 * C, from[i], 32 * C); });
   std::vector<uint16_t> erased;
   for (size_t i = 0; i < M; ++i)
     if (!known[i]) erased.push_back((uint16_t)i);
@@ -3087,9 +3239,9 @@ int zg_recover(zg_ctx* c, const uint64_t* row_ids, const uint8_t* const* rows, c
   if (!tm) return ZG_ERR_CUDA;
   k_rec_rows<<<(unsigned)k, 256, C * sizeof(Fr), s>>>(c->rec_rows, c->rec_ids, c->rec_V, lr, lc, c->tw.twi_c,
                                                        c->rec_ginv, c->tw.wni_lo, c->tw.wni_hi, c->rec_err);
-  k_rec_zinv<<<nblk(M, 128), 128, 0, s>>>(c->rec_erased, (uint32_t)erased.size(), c->rec_wpow, host_fr_from_u32(5),
+  k_rec_zinv<<<nblk(M, 32), 32 * REC_Z_WARPS, 0, s>>>(c->rec_erased, (uint32_t)erased.size(), c->rec_wpow, host_fr_from_u32(5),
                                           c->rec_zw, c->rec_zinv, (uint32_t)M);
-  k_rec_cols<<<(unsigned)C, 256, (M + R) * sizeof(Fr), s>>>(c->rec_V, c->rec_W, lr, lc, tm->twf_c, tm->twi_c,
+  k_rec_cols<<<(unsigned)C, REC_COL_THREADS, (M + R) * sizeof(Fr), s>>>(c->rec_V, c->rec_W, lr, lc, tm->twf_c, tm->twi_c,
                                                              c->rec_kpow, c->rec_kinv, c->rec_zw, c->rec_zinv, c->tw.twf_r,
                                                              c->tw.wn_lo, c->tw.wn_hi, c->rec_err);
   k_rec_out<<<(unsigned)R, 256, C * sizeof(Fr), s>>>(c->rec_W, c->rec_raw, lc, c->tw.twf_c, c->rec_err);
@@ -3109,7 +3261,7 @@ int zg_recover(zg_ctx* c, const uint64_t* row_ids, const uint8_t* const* rows, c
   for (size_t i = l32; i < c->max_raw; ++i)
     if (c->h_rec[i]) return fail(ZG_ERR_RECOVERY, "Non zero in padding range");
   if (out_cap < l32) return fail(ZG_ERR_INVALID_ARG, "output buffer too small");
-  memcpy(out, c->h_rec, l32);
+  host_copy(out, c->h_rec, l32);
   *out_len = l32;
   return ZG_OK;
 }
@@ -3119,14 +3271,18 @@ int zg_ctx_msm(zg_ctx* c, uint32_t coset, uint32_t line, const void* d_scalars, 
   if (!c->fb) return fail(ZG_ERR_INVALID_ARG, "zg_ctx_msm needs the fixed-base tables (msm_window_bits 0 or 11)");
   if (coset >= 3 || line >= (uint32_t)c->L) return fail(ZG_ERR_INVALID_ARG, "coset or line out of range");
   if (n < c->C || n > c->N || (n & (n - 1))) return fail(ZG_ERR_INVALID_ARG, "n must be a power of two in [2^log_col, N]");
-  // work items = chunks of 2^lcs points: 1024-point chunks leave most SMs
-  // idle below 2^19 points (one CTA per item), so chunks shrink down to 128
-  // points until there are 512 items, as far as the context's chunk buffers
-  // (3 R chunks) allow; the tables are per point, so any chunking reads them
   int logn = 0;
   while (((size_t)1 << logn) < n) ++logn;
-  int lcs = c->lc;
-  while (lcs > 7 && (n >> lcs) < 512 && (n >> (lcs - 1)) <= 3 * c->R) --lcs;
+  const uint32_t splits = fs_splits(logn);
+  // Few points: sorted in chunks of up to 1024, XYZZ additions in many short
+  // chains (k_fs_accum). More: work items of 2^lcs points for
+  // k_fb_accum. 1024-point chunks leave most SMs idle below 2^19 points (one
+  // CTA per item), so chunks shrink down to 128 points until there are 512
+  // items, as far as the context's chunk buffers (3 R chunks) allow; the
+  // tables are per point, so any chunking reads them
+  int lcs = splits ? std::min(logn, 10) : c->lc;
+  if (!splits)
+    while (lcs > 7 && (n >> lcs) < 512 && (n >> (lcs - 1)) <= 3 * c->R) --lcs;
   const int lrn = logn - lcs;
   const uint32_t nch = 1u << lrn;
   std::lock_guard<std::mutex> g(c->mu);
@@ -3135,23 +3291,28 @@ int zg_ctx_msm(zg_ctx* c, uint32_t coset, uint32_t line, const void* d_scalars, 
   ZG_CK(cudaStreamWaitEvent(s, c->done, 0));
   k_fb_sort<<<dim3(nch, 1), 256, fb_sort_smem_bytes(lcs), s>>>((const uint8_t*)d_scalars, c->lane.fb_offs, c->lane.fb_ents,
                                                                 lrn, lcs, 0, 0);
-  FbAccArgs fa;
-  fa.tab = c->line_ptr((int)coset, (int)line);
-  fa.offs = c->lane.fb_offs;
-  fa.ents = c->lane.fb_ents;
-  fa.out = c->lane.fb_out;
-  fa.ents32 = nullptr;
-  fa.lr = lrn;
-  fa.lc = lcs;
-  fa.lines = 1;
-  fa.l0 = 0;
-  fa.Ltot = 1;
-  fa.tabN = c->N;
-  launch_fb_accum(c, c->lane, c->msm_product, single_acc_plan(fa, nch), s);
-  launch_fb_combine(c->lane, single_fb_plan(lrn), s);
-  k_sum_points<<<1, 256, 0, s>>>(c->lane.part, nch, c->lane.nodes);
-  k_serialize_nodes<<<1, 128, 0, s>>>(c->lane.nodes, (uint8_t*)d_out, 1);
-  c->launches += 5;
+  if (splits) {
+    // (T, S) of every group and split go to the bucket kernel's scratch
+    XYZZ* ts = reinterpret_cast<XYZZ*>(c->lane.fb_scratch.base);
+    k_fs_accum<<<dim3(FS_CTAS, splits), 128, 0, s>>>(c->line_ptr((int)coset, (int)line), c->lane.fb_offs,
+                                                     c->lane.fb_ents, nch, lcs, (uint32_t)c->N, ts);
+    k_fs_combine<<<1, FS_COMBINE_THREADS, 0, s>>>(ts, splits, (uint8_t*)d_out);
+    c->launches += 3;
+  } else {
+    FbAccArgs fa;
+    fa.tab = c->line_ptr((int)coset, (int)line);
+    fa.offs = c->lane.fb_offs;
+    fa.ents = c->lane.fb_ents;
+    fa.out = c->lane.fb_out;
+    fa.lr = lrn;
+    fa.lc = lcs;
+    fa.tabN = c->N;
+    launch_fb_accum(c, c->lane, c->msm_product, single_acc_plan(fa, nch), s);
+    launch_fb_combine(c->lane, single_fb_plan(lrn), s);
+    const int sums = launch_sum_points(c->lane.part, nch, 0, 1, c->lane.nodes + 1, c->lane.nodes, s);
+    k_serialize_nodes<<<1, 128, 0, s>>>(c->lane.nodes, (uint8_t*)d_out, 1);
+    c->launches += 4 + sums;
+  }
   ZG_CK(cudaEventRecord(c->done, s));
   return check_launch();
 }
@@ -3451,17 +3612,11 @@ int zg_merkle_roots(const void* d_items, size_t n_items, void* d_roots, void* st
   if (per & (per - 1)) return fail(ZG_ERR_INVALID_ARG, "n_items must be 3*8*2^k");
   int depth = 0;
   while (((size_t)3 << depth) < leaves) ++depth;
-  std::vector<uint64_t> off(depth + 1);
-  size_t o = 0;
-  for (int d = 0; d <= depth; ++d) {
-    off[d] = o;
-    o += ((size_t)3 << d) * 32;
-  }
   cudaStream_t s = (cudaStream_t)stream;
   uint8_t* tree = nullptr;
   keep_pool_memory();
-  ZG_CK(cudaMallocAsync(&tree, o, s));
-  int rc = merkle_levels((const uint8_t*)d_items, n_items, tree, off, depth, s);
+  ZG_CK(cudaMallocAsync(&tree, 96 * (((size_t)2 << depth) - 1), s));
+  int rc = merkle_levels((const uint8_t*)d_items, n_items, tree, depth, s);
   if (!rc) ZG_CK(cudaMemcpyAsync(d_roots, tree, 96, cudaMemcpyDeviceToDevice, s));
   cudaFreeAsync(tree, s);
   return rc;

@@ -761,7 +761,18 @@ __global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __re
 
 }  // namespace zg
 #include "zg_bucket.cuh"
+#include "zg_quad.cuh"
 namespace zg {
+
+// a point as 64 bytes of ark G1 (16-byte aligned)
+__device__ __forceinline__ void store_g1(const XYZZ& p, uint8_t* out) {
+  uint8_t buf[64];
+  g1_serialize(p, buf);
+  uint4* d = reinterpret_cast<uint4*>(out);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(buf);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) d[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+}
 
 // Where a combine launch's items go. The launch covers up to FB_MAX_SETS item
 // sets (the chunk items, then one set per wide unit size); set k holds items
@@ -911,23 +922,216 @@ __global__ void __launch_bounds__(128) k_fb_combine_warp(const G1Aff* __restrict
   }
 }
 
-// out = sum of the n points of `in` (one CTA of 256 threads)
-__global__ void __launch_bounds__(256) k_sum_points(const XYZZ* __restrict__ in, uint32_t n, XYZZ* __restrict__ out) {
-  __shared__ XYZZ sh[256];
-  XYZZ acc = XYZZ::inf();
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) acc.add(load_xyzz(in + i));
-  sh[threadIdx.x] = acc;
+// ---------------------------------------------------------------------------
+// A single MSM over few points, where k_fb_accum's chain of tree levels and
+// shared inversions (30 us each) is the time: the chunks' sorted lists
+// (k_fb_sort) share one set of buckets, cut into groups of FS_BUCKETS, one CTA
+// of 128 threads per group and split. XYZZ additions: each thread sums the
+// entries of an even share of its group's list, the threads' partial sums of
+// a bucket meet in shared memory by quads, and the group's sums S = sum B_i,
+// T = sum (i + 1) B_i follow by a suffix sum of eight quads. The top window's
+// digits are 0, 1 or 2 (scalars below r), so its entries in buckets 0 and 1
+// (half the points) go to FS_TOP extra CTAs per split instead of making group
+// 0 the last to finish.
+// Whole MSM of 2^10 / 2^12 / 2^14 / 2^15 points: 0.23 / 0.36 / 0.50 / 0.73 ms,
+// against 0.75 / 0.75 / 0.76 / 0.93 by k_fb_accum; from 2^16 on the affine
+// additions win (1.24 against 1.47 ms at 2^16).
+constexpr int FS_BUCKETS = 8;
+constexpr int FS_GROUPS = FB_BUCKETS / FS_BUCKETS;  // 128
+constexpr int FS_TOP = 16;                          // CTAs for the top window, per split
+constexpr int FS_CTAS = FS_GROUPS + FS_TOP;
+// out[(split * FS_CTAS + cta) * 2 + {0, 1}] = {T, S} of a group, or of a share
+// of the top window's entries (whose buckets are group 0's). Split s takes
+// chunks s, s + splits, ..
+__global__ void __launch_bounds__(128, 4) k_fs_accum(const G1Aff* __restrict__ tab, const uint32_t* __restrict__ offs,
+                                                     const uint16_t* __restrict__ ents, uint32_t nch, int lc,
+                                                     uint32_t tabN, XYZZ* __restrict__ out) {
+  __shared__ __align__(16) XYZZ part[128];
+  __shared__ uint32_t first[FS_BUCKETS + 1];  // partial sums of bucket i: part[first[i]] .. part[first[i + 1] - 1]
+  const uint32_t tid = threadIdx.x, splits = gridDim.y;
+  const bool top = blockIdx.x >= FS_GROUPS;
+  const uint32_t k0 = top ? 0 : blockIdx.x * FS_BUCKETS;
+  // threads per bucket in proportion to its entries (top CTAs: buckets 0 and 1)
+  {
+    uint32_t n = 0;  // of bucket tid / 16, every 16th chunk of the split
+    const uint32_t i = tid >> 4;
+    if (!top || i < 2)
+      for (uint32_t g = blockIdx.y + (tid & 15) * splits; g < nch; g += 16 * splits) {
+        const uint32_t* o = offs + (size_t)g * (FB_BUCKETS + 1) + k0 + i;
+        n += o[1] - o[0];
+      }
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) n += __shfl_xor_sync(0xffffffffu, n, m);
+    if ((tid & 15) == 0) first[i] = n;
+  }
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      XYZZ t = sh[threadIdx.x];
-      t.add(sh[threadIdx.x + w]);
-      sh[threadIdx.x] = t;
+  if (tid == 0) {
+    uint32_t n[FS_BUCKETS], all = 0, nz = 0, at = 0;
+#pragma unroll
+    for (int i = 0; i < FS_BUCKETS; ++i) {
+      n[i] = first[i];
+      all += n[i];
+      nz += n[i] > 0;
+    }
+    // one thread per nonempty bucket, the rest in proportion
+#pragma unroll
+    for (int i = 0; i < FS_BUCKETS; ++i) {
+      first[i] = at;
+      if (n[i]) at += 1 + (uint32_t)((uint64_t)n[i] * (128 - nz) / all);
+    }
+    first[FS_BUCKETS] = at;
+  }
+  __syncthreads();
+  uint32_t b = 0;
+  while (b + 1 < FS_BUCKETS && tid >= first[b + 1]) ++b;
+  const uint32_t lanes = first[b + 1] - first[b], lane = tid - first[b];
+  XYZZ acc = XYZZ::inf();
+  if (tid < first[FS_BUCKETS]) {
+    const uint32_t share = top ? (blockIdx.x - FS_GROUPS) * lanes + lane : lane, shares = top ? FS_TOP * lanes : lanes;
+    uint32_t at = share;  // position in the bucket's list, over all chunks
+    G1Aff next = aff_inf();  // loaded behind the addition before it
+    for (uint32_t g = blockIdx.y; g < nch; g += splits) {
+      const uint32_t* o = offs + (size_t)g * (FB_BUCKETS + 1) + k0 + b;
+      const uint32_t e0 = o[0], n = o[1] - e0;
+      const uint16_t* list = ents + (size_t)g * FB_WINDOWS * (1u << lc) + e0;
+      const G1Aff* tg = tab + ((size_t)g << lc);
+      for (; at < n; at += shares) {
+        const uint32_t v = list[at], w = (v >> 10) & 31;
+        if ((w == FB_WINDOWS - 1 && k0 + b < 2) != top) continue;
+        G1Aff p = ld_aff(tg + (size_t)w * tabN + (v & 0x3ff));
+        if (v >> 15) p.y = -p.y;
+        if (!aff_is_inf(next)) acc.add_affine(next.x, next.y);
+        next = p;
+      }
+      at -= n;
+    }
+    if (!aff_is_inf(next)) acc.add_affine(next.x, next.y);
+  }
+  store_xyzz(part + tid, acc);
+  __syncthreads();
+  // each bucket's partial sums by pairs, in place from first[i] on: the pairs
+  // of all buckets of a step share the 32 quads
+  const uint32_t quad = tid >> 2;
+  for (uint32_t step = 0;; ++step) {
+    uint32_t pairs = 0, most = 0;
+#pragma unroll
+    for (int i = 0; i < FS_BUCKETS; ++i) {
+      const uint32_t n = (first[i + 1] - first[i] + (1u << step) - 1) >> step;
+      pairs += n >> 1;
+      most = max(most, n);
+    }
+    if (most <= 1) break;
+    for (uint32_t j0 = 0; j0 < pairs; j0 += 32) {  // at most two rounds
+      uint32_t j = j0 + quad, at = 0, odd = 0;
+      const bool there = j < pairs;
+#pragma unroll
+      for (int i = 0; i < FS_BUCKETS; ++i) {
+        const uint32_t n = (first[i + 1] - first[i] + (1u << step) - 1) >> step;
+        if (j < n >> 1) {
+          at = first[i] + (j << (step + 1));
+          odd = 1u << step;
+          break;
+        }
+        j -= n >> 1;
+      }
+      const Fq x = there ? quad_load(part + at) : quad_inf(), y = there ? quad_load(part + at + odd) : quad_inf();
+      const Fq z = quad_add(x, y);
+      if (there) quad_store(part + at, z);  // a pair's places are its own
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) store_xyzz(out, sh[0]);
+  if (tid >= 32) return;
+  const uint32_t mine = first[quad + 1] > first[quad] ? first[quad] : 0;
+  Fq u = quad_load(part + mine);  // bucket `quad` of the group
+  u = quad_sel(first[quad + 1] > first[quad], u, quad_inf());
+#pragma unroll 1
+  for (int d = 1; d < 8; d <<= 1) {
+    const Fq x = quad_add(u, quad_down(u, d));
+    u = quad_sel((int)quad + d < 8, x, u);
+  }
+  const Fq t = quad_warp_sum(u);
+  XYZZ* o = out + ((size_t)blockIdx.y * FS_CTAS + blockIdx.x) * 2;
+  if (quad == 0) {
+    quad_store(o, t);
+    quad_store(o + 1, u);
+  }
 }
+// P = sum_c T_c + FS_BUCKETS sum_c c S_c over the groups c and all splits, the
+// top window's (T, S) at c = 0; serialized. One CTA of 64 quads, quad g takes
+// groups 2 g and 2 g + 1, suffix sums of the quads' S in shared memory.
+constexpr int FS_COMBINE_THREADS = 256;
+__global__ void __launch_bounds__(FS_COMBINE_THREADS) k_fs_combine(const XYZZ* __restrict__ in, uint32_t splits,
+                                                                   uint8_t* __restrict__ out) {
+  constexpr uint32_t Q = FS_COMBINE_THREADS / 4;
+  static_assert(FS_GROUPS == 2 * Q && FS_BUCKETS == 8, "two groups per quad, doublings below");
+  __shared__ __align__(16) XYZZ sh[Q];
+  const uint32_t g = threadIdx.x >> 2;
+  const XYZZ* p = in + (size_t)4 * g;
+  Fq t = quad_add(quad_load(p), quad_load(p + 2));
+  Fq w = quad_load(p + 3), run = quad_load(p + 1);  // S of groups 2 g + 1 and 2 g
+#pragma unroll 1
+  for (uint32_t s = 1; s < splits; ++s) {
+    p += 2 * FS_CTAS;
+    t = quad_add(t, quad_add(quad_load(p), quad_load(p + 2)));
+    w = quad_add(w, quad_load(p + 3));
+    run = quad_add(run, quad_load(p + 1));
+  }
+  run = quad_add(run, w);
+  // the top window's T (its S has weight 0)
+#pragma unroll 1
+  for (uint32_t k = g; k < ((splits * FS_TOP + Q - 1) & ~(Q - 1)); k += Q) {
+    const bool there = k < splits * FS_TOP;
+    const Fq x = quad_load(in + ((size_t)(there ? k / FS_TOP : 0) * FS_CTAS + FS_GROUPS + k % FS_TOP) * 2);
+    t = quad_add(t, quad_sel(there, x, quad_inf()));
+  }
+  // U_g = sum_{m >= g} run_m over the quads
+#pragma unroll 1
+  for (uint32_t d = 1; d < Q; d <<= 1) {
+    __syncthreads();
+    quad_store(sh + g, run);
+    __syncthreads();
+    const Fq x = quad_load(sh + min(g + d, Q - 1));
+    run = quad_add(run, quad_sel(g + d < Q, x, quad_inf()));
+  }
+  // sum_c c S_c = 2 sum_{g >= 1} U_g + sum_g w_g, times 8
+  Fq v = quad_add(quad_dbl(quad_sel(g >= 1, run, quad_inf())), w);
+  v = quad_dbl(quad_dbl(quad_dbl(v)));
+  v = quad_warp_sum(quad_add(v, t));
+  __syncthreads();
+  if ((g & 7) == 0) quad_store(sh + g / 8, v);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  v = quad_warp_sum(quad_load(sh + g));
+  __syncwarp();
+  if (g == 0) quad_store(sh, v);
+  __syncwarp();
+  if (threadIdx.x == 0) store_g1(sh[0], out);
+}
+
+// out[y * gridDim.x + x] = sum of points x, x + gridDim.x, .. of the n at in +
+// y stride, by quads (64 per CTA): n / (64 gridDim.x) additions in a row and
+// six of the tree. launch_sum_points picks the grid.
+constexpr int SUM_THREADS = 256;
+__global__ void __launch_bounds__(SUM_THREADS) k_sum_points(const XYZZ* __restrict__ in, uint32_t n, uint64_t stride,
+                                                            XYZZ* __restrict__ out) {
+  __shared__ __align__(16) XYZZ sh[SUM_THREADS / 32];
+  in += blockIdx.y * stride;
+  const uint32_t quads = gridDim.x * (SUM_THREADS / 4);
+  Fq acc = quad_inf();
+  // the loop's bound is uniform per CTA: all lanes of a warp add together
+  for (uint32_t base = blockIdx.x * (SUM_THREADS / 4); base < n; base += quads) {
+    const uint32_t i = base + threadIdx.x / 4;
+    acc = quad_add(acc, i < n ? quad_load(in + i) : quad_inf());
+  }
+  acc = quad_warp_sum(acc);
+  if ((threadIdx.x & 31) < 4) quad_store(sh + threadIdx.x / 32, acc);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    acc = quad_warp_sum(quad_load(sh + threadIdx.x / 4));
+    if (threadIdx.x < 4) quad_store(out + blockIdx.y * gridDim.x + blockIdx.x, acc);
+  }
+}
+static_assert(SUM_THREADS == 256, "one partial per quad of the last warp");
 
 // sum_w 2^{8w} win[w] for each (coset, line, chunk)
 __global__ void __launch_bounds__(64) k_msm_combine(const XYZZ* __restrict__ win, XYZZ* __restrict__ out, uint32_t count) {
@@ -951,115 +1155,138 @@ __global__ void __launch_bounds__(64) k_msm_combine(const XYZZ* __restrict__ win
 __device__ __forceinline__ uint32_t amt_commit_off(int d) { return 1 + ((2u << d) - 2); }
 __device__ __forceinline__ uint32_t amt_proof_off(int d, int lr) { return (2u << lr) - 1 + ((2u << d) - 2); }
 
-__global__ void __launch_bounds__(256) k_amt_tree(XYZZ* __restrict__ part, XYZZ* __restrict__ nodes, int lr, int lines) {
+// Levels of few nodes are a chain of dependent additions, so the nodes are
+// added by quads (zg_quad.cuh): 128 parts per line take 24 us, 85 with one lane
+// per node.
+constexpr int AMT_THREADS = 512;
+__global__ void __launch_bounds__(AMT_THREADS) k_amt_tree(XYZZ* __restrict__ part, XYZZ* __restrict__ nodes, int lr,
+                                                          int lines) {
   const int l = blockIdx.x, c = blockIdx.y;
   const int R = 1 << lr;
   const uint32_t per_coset = 4u * R - 2;
   XYZZ* p = part + ((size_t)c * lines + l) * R;
   XYZZ* o = nodes + (size_t)c * per_coset;
+  const int quad = threadIdx.x >> 2, quads = blockDim.x >> 2;
+  auto copy = [&](XYZZ* dst, int n) {
+    for (int i = quad; i < n; i += quads) quad_store(dst + i, quad_load(p + i));
+  };
   // levels to reduce: quotient layer d = l + 1 keeps 2^d nodes; basis keeps all
   // levels; high keeps 1
   int keep_log = (l < lr) ? (l + 1) : 0;
   const bool is_basis = (l == lr);
-  if (is_basis) {
-    for (int i = threadIdx.x; i < R; i += blockDim.x) o[amt_commit_off(lr - 1) + i] = p[i];
-  }
+  if (is_basis) copy(o + amt_commit_off(lr - 1), R);
   int cur = R;
   int lvl = lr;  // current array holds 2^lvl nodes
   while (lvl > keep_log) {
     int half = cur >> 1;
     __syncthreads();
     // read pairs then write, two phases to allow in-place reduction
-    for (int base = 0; base < half; base += blockDim.x) {
-      int i = base + threadIdx.x;
-      XYZZ s;
-      if (i < half) {
-        s = p[2 * i];
-        s.add(p[2 * i + 1]);
-      }
+    for (int base = 0; base < half; base += quads) {
+      const int i = base + quad;
+      const Fq a = i < half ? quad_load(p + 2 * i) : quad_inf(), b = i < half ? quad_load(p + 2 * i + 1) : quad_inf();
+      Fq s = quad_inf();
+      if (base + (int)(threadIdx.x & ~31u) / 4 < half) s = quad_add(a, b);  // uniform per warp
       __syncthreads();
-      if (i < half) p[i] = s;
+      if (i < half) quad_store(p + i, s);
       __syncthreads();
     }
     cur = half;
     --lvl;
-    if (is_basis) {
-      if (lvl >= 1) {
-        for (int i = threadIdx.x; i < cur; i += blockDim.x) o[amt_commit_off(lvl - 1) + i] = p[i];
-      } else if (threadIdx.x == 0) {
-        o[0] = p[0];
-      }
-    }
+    if (is_basis) copy(lvl >= 1 ? o + amt_commit_off(lvl - 1) : o, cur);
   }
   __syncthreads();
-  if (l < lr) {
-    for (int i = threadIdx.x; i < cur; i += blockDim.x) o[amt_proof_off(l, lr) + i] = p[i];
-  } else if (l == lr + 1) {
-    if (threadIdx.x == 0) o[per_coset - 1] = p[0];
-  }
+  if (l < lr) copy(o + amt_proof_off(l, lr), cur);
+  else if (l == lr + 1) copy(o + per_coset - 1, 1);
 }
 
 // XYZZ node -> 64-byte ark G1
 __global__ void __launch_bounds__(128) k_serialize_nodes(const XYZZ* __restrict__ nodes, uint8_t* __restrict__ out, uint32_t count) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  uint8_t buf[64];
-  g1_serialize(nodes[i], buf);
-  uint4* d = reinterpret_cast<uint4*>(out + (size_t)i * 64);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(buf);
-  d[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  d[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  d[2] = make_uint4(w[8], w[9], w[10], w[11]);
-  d[3] = make_uint4(w[12], w[13], w[14], w[15]);
+  if (i < count) store_g1(nodes[i], out + (size_t)i * 64);
 }
 
 // ---------------------------------------------------------------------------
 // Merkle tree (merkle/blob.rs:15-34): leaves = keccak(8 x 32 B), parents =
-// keccak(left || right) until 3 coset roots remain.
-__global__ void __launch_bounds__(128) k_merkle_leaves(const uint8_t* __restrict__ data, uint8_t* __restrict__ leaves, uint32_t count) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const uint64_t* src = reinterpret_cast<const uint64_t*>(data + (size_t)i * 256);
-  uint64_t in[32];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    ulonglong2 v = reinterpret_cast<const ulonglong2*>(src)[k];
-    in[2 * k] = v.x;
-    in[2 * k + 1] = v.y;
-  }
-  uint64_t out[4];
-  keccak256_256(in, out);
-  ulonglong2* d = reinterpret_cast<ulonglong2*>(leaves + (size_t)i * 32);
-  d[0] = make_ulonglong2(out[0], out[1]);
-  d[1] = make_ulonglong2(out[2], out[3]);
+// keccak(left || right) until 3 coset roots remain. Level d holds 3 * 2^d
+// nodes (coset c's at c 2^d ..), at byte offset 96 (2^d - 1) of the tree
+// buffer, so a level's nodes pair up across the whole level alike.
+constexpr int MERKLE_THREADS = 128;
+__device__ __forceinline__ uint8_t* merkle_level(uint8_t* tree, int d) { return tree + 96 * ((1ull << d) - 1); }
+__device__ __forceinline__ void merkle_store(uint8_t* level, size_t i, const uint64_t h[4]) {
+  ulonglong2* o = reinterpret_cast<ulonglong2*>(level + i * 32);
+  o[0] = make_ulonglong2(h[0], h[1]);
+  o[1] = make_ulonglong2(h[2], h[3]);
 }
-__global__ void __launch_bounds__(128) k_merkle_parents(const uint8_t* __restrict__ child, uint8_t* __restrict__ parent, uint32_t count) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const ulonglong2* src = reinterpret_cast<const ulonglong2*>(child + (size_t)i * 64);
-  uint64_t in[8];
+// The CTA's nodes (one per thread, h, of level d) and their ancestors up to
+// `up` levels above: each level is hashed from the previous one in shared
+// memory and written out: levels of few nodes are bounded by the latency of
+// one permutation each (7.4 us), and the gaps between launches go.
+__device__ __forceinline__ void merkle_ancestors(uint8_t* tree, int d, int up, uint64_t h[4]) {
+  __shared__ uint64_t sn[MERKLE_THREADS * 4];
+  for (int u = 1; u <= up; ++u) {
+    if (u > 1) __syncthreads();
+    if (threadIdx.x < (unsigned)MERKLE_THREADS >> (u - 1))
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sn[4 * threadIdx.x + k] = h[k];
+    __syncthreads();
+    if (threadIdx.x < (unsigned)MERKLE_THREADS >> u) {
+      uint64_t in[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) in[k] = sn[8 * threadIdx.x + k];
+      keccak256_64(in, h);
+      merkle_store(merkle_level(tree, d - u), (size_t)blockIdx.x * (MERKLE_THREADS >> u) + threadIdx.x, h);
+    }
+  }
+}
+// The leaves, level `depth`. The CTA's 128 leaves of 256 bytes come in by
+// cp.async, coalesced, to rows of 272 bytes (16 of padding: a thread's 16-byte
+// reads of its own row spread over the banks), so the second block of a leaf
+// stays in shared memory during the first permutation (78 registers, 103 before).
+constexpr int MERKLE_ROW = 17;  // 16-byte words per staged leaf
+__global__ void __launch_bounds__(MERKLE_THREADS, 6) k_merkle_leaves(const uint8_t* __restrict__ data,
+                                                                     uint8_t* __restrict__ tree, int depth,
+                                                                     uint32_t count) {
+  __shared__ uint4 rows[MERKLE_THREADS * MERKLE_ROW];
+  const uint32_t i0 = blockIdx.x * MERKLE_THREADS, here = min((uint32_t)MERKLE_THREADS, count - i0);
+  const uint4* src = reinterpret_cast<const uint4*>(data) + (size_t)i0 * 16;
+  for (uint32_t k = threadIdx.x; k < here * 16; k += MERKLE_THREADS) cp16(rows + (k >> 4) * MERKLE_ROW + (k & 15), src + k);
+  cp_commit();
+  cp_wait<0>();
+  __syncthreads();
+  if (threadIdx.x >= here) return;
+  const uint4* row = rows + threadIdx.x * MERKLE_ROW;
+  uint64_t h[4];
+  keccak256_256([&](int k) {
+    const uint4 v = row[k];
+    return make_ulonglong2((uint64_t)v.y << 32 | v.x, (uint64_t)v.w << 32 | v.z);
+  }, h);
+  merkle_store(merkle_level(tree, depth), i0 + threadIdx.x, h);
+}
+// levels d - 1 .. d - 1 - up from level d (3 * 2^d a multiple of 256): a CTA
+// takes 256 nodes
+__global__ void __launch_bounds__(MERKLE_THREADS) k_merkle_parents(uint8_t* __restrict__ tree, int d, int up) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const ulonglong2* src = reinterpret_cast<const ulonglong2*>(merkle_level(tree, d) + (size_t)i * 64);
+  uint64_t in[8], h[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     ulonglong2 v = src[k];
     in[2 * k] = v.x;
     in[2 * k + 1] = v.y;
   }
-  uint64_t out[4];
-  keccak256_64(in, out);
-  ulonglong2* d = reinterpret_cast<ulonglong2*>(parent + (size_t)i * 32);
-  d[0] = make_ulonglong2(out[0], out[1]);
-  d[1] = make_ulonglong2(out[2], out[3]);
+  keccak256_64(in, h);
+  merkle_store(merkle_level(tree, d - 1), i, h);
+  merkle_ancestors(tree, d - 1, up, h);
 }
-// The upper levels of the Merkle tree in one launch: levels top - 1 .. 0
-// from level top (at most 1024 nodes per coset), one CTA per coset subtree,
-// each level hashed from the previous one in shared memory and written out.
-// Level d holds 3 * 2^d nodes (coset c's at c 2^d ..), at byte offset
-// 96 (2^d - 1) of the tree buffer. Block size max(1, 2^(top - 1)).
-constexpr int MERKLE_TOP_MAX = 10;
-__global__ void __launch_bounds__(512) k_merkle_top(uint8_t* __restrict__ tree, int top) {
+// The upper levels of the tree in one launch: levels top - 1 .. 0 from level
+// top (at most 2^MERKLE_TOP_MAX nodes per coset), one CTA per coset subtree.
+// Block size max(1, 2^(top - 1)). 512 nodes per coset are two warps per
+// scheduler at the first level, about one permutation's latency.
+constexpr int MERKLE_TOP_MAX = 9;
+__global__ void __launch_bounds__(256) k_merkle_top(uint8_t* __restrict__ tree, int top) {
   __shared__ uint64_t sn[(1 << MERKLE_TOP_MAX) * 4];
   const uint32_t c = blockIdx.x, n = 1u << top;
-  const uint64_t* src = reinterpret_cast<const uint64_t*>(tree + 96 * ((1ull << top) - 1) + (size_t)c * n * 32);
+  const uint64_t* src = reinterpret_cast<const uint64_t*>(merkle_level(tree, top) + (size_t)c * n * 32);
   for (uint32_t i = threadIdx.x; i < 4 * n; i += blockDim.x) sn[i] = src[i];
   __syncthreads();
   for (int d = top - 1; d >= 0; --d) {
@@ -1073,7 +1300,7 @@ __global__ void __launch_bounds__(512) k_merkle_top(uint8_t* __restrict__ tree, 
     }
     __syncthreads();
     if (i < cnt) {
-      uint64_t* dst = reinterpret_cast<uint64_t*>(tree + 96 * ((1ull << d) - 1) + ((size_t)c * cnt + i) * 32);
+      uint64_t* dst = reinterpret_cast<uint64_t*>(merkle_level(tree, d) + ((size_t)c * cnt + i) * 32);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         sn[4 * i + k] = out[k];

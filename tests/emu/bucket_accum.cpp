@@ -46,9 +46,9 @@ int main(int argc, char** argv) {
   const int lc = kind == "small" ? 5 : 10, ulog = 11, mlog = kind == "merged" || kind == "skewed" ? 1 : 0;
   const uint32_t units = 1u << mlog, unit_points = wide ? 1u << ulog : 1u << lc, buckets = wide ? 1u << ulog : 1024u;
   const uint32_t points = unit_points * units, W = wide ? (uint32_t)wd_windows(ulog) : FB_WINDOWS;
-  const uint32_t items = wide ? buckets / 1024 : 1;
+  const uint32_t items = wide ? buckets / 1024 : 1;  // of the same lists for every line
   const std::vector<G1Aff> base = multiples(300);
-  std::vector<G1Aff> tab((size_t)W * points);
+  std::vector<G1Aff> tab((size_t)3 * W * points);
   for (G1Aff& p : tab) {
     p = base[rng() % base.size()];
     if (rng() % 2) p.y = -p.y;
@@ -79,9 +79,10 @@ int main(int argc, char** argv) {
     offs.push_back(at);
   }
   FbAccPlan plan;
-  std::vector<G1Aff> out((size_t)items * FB_OUT);
+  const uint32_t lines = 3;  // table lines that read the same lists
+  std::vector<G1Aff> out((size_t)items * lines * FB_OUT);
   plan.n = 1;
-  plan.start[1] = items;
+  plan.start[1] = items * lines;
   FbAccArgs& a = plan.a[0];
   a.tab = tab.data();
   a.offs = offs.data();
@@ -93,23 +94,26 @@ int main(int argc, char** argv) {
   a.ulog = ulog;
   a.mlog = mlog;
   a.W = (int)W;
+  a.lines = a.Ltot = (int)lines;
   a.tabN = points;
+  a.group = (int)group;
   FbScratch s;
-  s.cap = kind == "skewed" ? 8192 : 2 * W * 1536 << mlog;
+  s.cap = kind == "skewed" ? 8192 : min(FB_GROUP * W * 1536 << mlog, FB_CAP_MAX);
   std::vector<uint8_t> mem(s.bytes() + 256);
   s.base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mem.data()) + 255) / 256 * 256);
   uint32_t next = 0;
-  run_block(FB_ACC_THREADS, [&] { k_fb_accum<MulImad>(plan, s, &next, 32, group); });
+  run_block(FB_ACC_THREADS, [&] { k_fb_accum<MulImad>(plan, s, &next, 32); });
 
   int bad = 0;
-  for (uint32_t it = 0; it < items; ++it) {
+  for (uint32_t item = 0; item < items * lines; ++item) {
+    const uint32_t it = item / lines, line = item % lines;
     std::vector<XYZZ> sum(1024, XYZZ::inf());
     for (uint32_t u = 0; u < units; ++u)
       for (uint32_t k = 0; k < 1024; ++k)
         for (uint32_t v : list[(size_t)u * buckets + it * 1024 + k]) {
           const uint32_t lg = wide ? (uint32_t)ulog : 10u;
           const uint32_t idx = (v & ((1u << lg) - 1)) + u * unit_points, w = (v >> lg) & 31;
-          G1Aff q = tab[(size_t)w * points + idx];
+          G1Aff q = tab[((size_t)line * W + w) * points + idx];
           if (wide ? v >> 31 : (v >> 15) & 1) q.y = -q.y;
           sum[k].add_affine(q.x, q.y);
         }
@@ -119,9 +123,9 @@ int main(int argc, char** argv) {
         row.add(sum[32 * r + c]);
         col.add(sum[32 * c + r]);
       }
-      bad += !same(row, out[it * FB_OUT + r]) + !same(col, out[it * FB_OUT + 32 + r]);
+      bad += !same(row, out[item * FB_OUT + r]) + !same(col, out[item * FB_OUT + 32 + r]);
     }
   }
-  printf("%s: %d of %u sums differ\n", kind.c_str(), bad, items * FB_OUT);
+  printf("%s: %d of %u sums differ\n", kind.c_str(), bad, items * lines * FB_OUT);
   return bad != 0;
 }

@@ -24,8 +24,8 @@ def runner(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("kind,group", [("chunk", 1), ("small", 2), ("wide", 1), ("wide", 2), ("merged", 1),
-                                        ("merged", 2), ("skewed", 2), ("empty", 1)])
+@pytest.mark.parametrize("kind,group", [("chunk", 1), ("chunk", 3), ("small", 2), ("small", 3), ("wide", 1),
+                                        ("wide", 4), ("merged", 2), ("skewed", 1), ("skewed", 4), ("empty", 2)])
 def test_bucket_sums(runner, kind, group):
     r = subprocess.run([runner, kind, str(group), "11"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr

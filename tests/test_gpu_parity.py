@@ -690,3 +690,53 @@ def test_encode_matches_golden_fixture(gpu_pkg, fixture):
     assert hashlib.sha256(reply.encoded_data).hexdigest() == g["encoded_data_sha256"]
     assert [hashlib.sha256(s).hexdigest() for s in reply.encoded_slice] == g["slice_sha256"]
     params.close()
+
+
+@pytest.fixture(scope="module")
+def ctx_6x10(gpu_pkg):
+    params = gpu_pkg.ZgEncoderParams.from_seed(6, 10, 21)
+    yield params
+    params.close()
+
+
+@pytest.mark.parametrize("log_n,kind", [(10, "uniform"), (12, "uniform"), (12, "top"), (12, "zero"), (14, "equal"),
+                                        (15, "uniform"), (16, "uniform")])
+def test_ctx_msm_paths_match_oracle(gpu_pkg, oracle, ctx_6x10, log_n, kind):
+    """Single MSMs on both sides of the size where zg_ctx_msm changes kernels
+    (up to 2^15 points XYZZ sums of bucket groups, above it the affine bucket
+    kernel): one split and several, every top-window digit, no entries at all,
+    and equal scalars (a few buckets hold everything)."""
+    n = 1 << log_n
+    rng = np.random.default_rng(log_n)
+    if kind == "zero":
+        scal = bytes(32 * n)
+    elif kind == "equal":
+        scal = ((0x1234567 << 200) + 77).to_bytes(32, "little") * n
+    else:
+        scal = bytearray(rand_fr_bytes(rng, n))
+        if kind == "top":  # digits 0, 1 and 2 of the top window, with and without carries
+            for i in range(0, n, 3):
+                v = R_MOD - 1 - int(rng.integers(0, 1 << 62)) if i % 2 else (1 << 253) - 1 - i
+                scal[32 * i:32 * i + 32] = v.to_bytes(32, "little")
+        scal = bytes(scal)
+    bases = ctx_6x10.param_line(1, 6, 0, n)
+    out = empty(64)
+    ts = dev(scal)
+    rc = gpu_pkg.lib().zg_ctx_msm(ctx_6x10.handle, 1, 6, ts.data_ptr(), n, out.data_ptr(), None)
+    assert rc == 0, gpu_pkg.lib().zg_last_error()
+    assert host(out) == oracle.msm(bases, scal)
+
+
+@pytest.mark.parametrize("log_per_root", [0, 1, 5, 9, 10, 12, 13, 15, 16])
+def test_merkle_levels_match_oracle(gpu_pkg, oracle, log_per_root):
+    """Merkle roots at depths on every side of the launch plan: the top kernel
+    alone, with one to three fused levels below it, and with single levels."""
+    n = 24 << log_per_root
+    items = rand_fr_bytes(np.random.default_rng(log_per_root), n)
+    out = empty(96)
+    ti = dev(items)
+    rc = gpu_pkg.lib().zg_merkle_roots(ti.data_ptr(), n, out.data_ptr(), None)
+    assert rc == 0, gpu_pkg.lib().zg_last_error()
+    # 3 roots of 2^k leaves of 8 items: a blob of 2^(k - 4) rows of 128 columns has the same tree
+    lr, lc = (log_per_root, 3) if log_per_root < 8 else (log_per_root - 7, 10)
+    assert host(out) == oracle.merkle_roots(lr, lc, items)
