@@ -107,6 +107,9 @@ struct Twiddles {
   Fr *twf_c = nullptr, *twi_c = nullptr, *twf_r = nullptr, *twi_r = nullptr;
   Fr *wn_lo = nullptr, *wn_hi = nullptr, *wni_lo = nullptr, *wni_hi = nullptr;
   Fr *gs_lo = nullptr, *gs_hi = nullptr;  // coset scale tables (cosets 1, 2)
+  // the column pass's factors in its own order, [column][row], for zg_ntt:
+  // w_N^(s r) and w_N^(-s r) / N
+  Fr *wn_full = nullptr, *wni_full = nullptr;
 };
 
 template <class T>
@@ -163,7 +166,7 @@ int make_twiddles(int lr, int lc, Twiddles* tw) {
 }
 void free_twiddles(Twiddles* tw) {
   Fr* ps[] = {tw->twf_c, tw->twi_c, tw->twf_r, tw->twi_r, tw->wn_lo, tw->wn_hi,
-              tw->wni_lo, tw->wni_hi, tw->gs_lo, tw->gs_hi};
+              tw->wni_lo, tw->wni_hi, tw->gs_lo, tw->gs_hi, tw->wn_full, tw->wni_full};
   for (Fr* p : ps) if (p) cudaFree(p);
   *tw = Twiddles();
 }
@@ -207,24 +210,29 @@ int set_smem_limits() {
 
 inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
-// threads of a CTA that runs one 2^logn-point transform: one per radix-4
-// group of the shared-memory passes (2^(logn - 2)), within [32, 256]
+// threads of a CTA that runs one 2^logn-point transform: one per radix-4 group
+// of the shared-memory passes (2^(logn - 2)), at most 256. Fewer threads with
+// more groups each would let more CTAs of a small transform share an SM, but
+// the serial chain of products per thread is what the passes wait for: 1024
+// transforms of 2^10 took 105 us with 256 threads, 108 with 128, 125 with 64,
+// one inverse of 2^20 209, 230 and 280 us.
 unsigned ntt_threads(int logn) { return (unsigned)std::min(256, std::max(32, 1 << std::max(0, logn - 2))); }
 
 // natural-order N-point transform out = DFT(x) (or inverse without 1/N), via
 // the column / row passes; tmp has N elements
-// (batch vectors back to back in x, tmp and out; batch <= 65535). With cs_lo
-// set, input i is first multiplied by g^i = cs_lo[i mod 2^cs_h] cs_hi[i >> cs_h]
-// (coset shift); with scale set, every output by *scale.
+// (batch vectors back to back in x, tmp and out; batch <= 65535). With cs
+// set, input q C + s of each vector is first multiplied by cs[s R + q] (coset
+// shift). wfull: w_N^(+-s r) in the column pass's order, scale included, or
+// null (products of the two power tables).
 void ntt4(const Twiddles& tw, const Fr* x, Fr* tmp, Fr* out, bool inverse, cudaStream_t s, uint32_t batch = 1,
-          const Fr* cs_lo = nullptr, const Fr* cs_hi = nullptr, int cs_h = 0, const Fr* scale = nullptr) {
+          const Fr* wfull = nullptr, const Fr* cs = nullptr) {
   const int lr = tw.lr, lc = tw.lc;
   const size_t R = size_t(1) << lr, C = size_t(1) << lc;
   k_ntt4_colpass<<<dim3((unsigned)C, batch), ntt_threads(lr), R * sizeof(Fr), s>>>(
       x, tmp, lr, lc, inverse ? tw.twi_r : tw.twf_r, inverse ? tw.wni_lo : tw.wn_lo, inverse ? tw.wni_hi : tw.wn_hi,
-      cs_lo, cs_hi, cs_h);
+      wfull, cs);
   k_ntt4_rowpass<<<dim3((unsigned)R, batch), ntt_threads(lc), C * sizeof(Fr), s>>>(
-      tmp, out, lr, lc, inverse ? tw.twi_c : tw.twf_c, scale != nullptr, scale ? *scale : Fr::zero());
+      tmp, out, lr, lc, inverse ? tw.twi_c : tw.twf_c);
 }
 
 }  // namespace
@@ -1242,41 +1250,69 @@ const Twiddles* cached_twiddles(int lr, int lc) {
   return &(g_ntt_tw[key] = t);
 }
 
-// g^e for e < 2^logn as lo[e & (2^h - 1)] * hi[e >> h], h = (logn + 1) / 2
-// (Montgomery form), for the coset shift of zg_ntt; one pair per (device, logn,
-// coset)
-// g^e = lo[e mod 2^h] * hi[e >> h] for e < 2^logn (h = logn: lo alone)
-struct CosetPows {
-  Fr* lo = nullptr;
-  Fr* hi = nullptr;
-  int h = 0;
-};
-std::map<std::tuple<int, int, uint32_t>, CosetPows> g_coset_pows;  // per device; guarded by g_ntt_mu
+// Factor tables of the standalone transforms, built on the device on their
+// first use and kept for the process: out[s R + r] = base^(s r) scale
+// (`shift` false) or base^(r C + s) (true), from the split power tables lo[C]
+// and hi[R] of base.
+int build_full_table(const Fr* lo, const Fr* hi, int lr, int lc, bool shift, const Fr& scale, Fr** out) {
+  const size_t N = size_t(1) << (lr + lc);
+  Fr* t = nullptr;
+  ZG_CK(cudaMalloc(&t, N * sizeof(Fr)));
+  cudaStream_t s = nullptr;
+  bool ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  if (ok) {
+    k_full_table<<<nblk(N, 256), 256, 0, s>>>(lo, hi, lr, lc, shift ? 1 : 0, scale, t);
+    ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+    cudaStreamDestroy(s);
+  }
+  if (!ok) {
+    cudaFree(t);
+    return fail(ZG_ERR_CUDA, "transform table build failed");
+  }
+  *out = t;
+  return 0;
+}
 
-const CosetPows* cached_coset_pows(int logn, uint32_t coset) {
+// the coset factors g^i of zg_ntt per (device, logn, coset): i < 2^logn in
+// order up to the single-CTA transform's size, in the column pass's order
+// above it
+std::map<std::tuple<int, int, uint32_t>, Fr*> g_coset_pows;  // guarded by g_ntt_mu
+
+const Fr* cached_coset_pows(int logn, uint32_t coset) {
   std::lock_guard<std::mutex> g(g_ntt_mu);
   auto key = std::make_tuple(current_device(), logn, coset);
   auto it = g_coset_pows.find(key);
-  if (it != g_coset_pows.end()) return &it->second;
-  CosetPows p;
-  // one full table up to the single-CTA transform's size, else split in two
-  p.h = logn <= 11 ? logn : (logn + 1) / 2;
-  const size_t nlo = size_t(1) << p.h, nhi = size_t(1) << (logn - p.h);
+  if (it != g_coset_pows.end()) return it->second;
   const Fr gen = coset_factor(logn, coset);
-  std::vector<Fr> lo(nlo), hi(nhi);
-  lo[0] = Fr::one();
-  for (size_t j = 1; j < nlo; ++j) lo[j] = lo[j - 1] * gen;
-  const Fr gh = lo[nlo - 1] * gen;  // g^(2^h)
-  hi[0] = Fr::one();
-  for (size_t j = 1; j < nhi; ++j) hi[j] = hi[j - 1] * gh;
-  if (cudaMalloc(&p.lo, nlo * sizeof(Fr)) != cudaSuccess || cudaMalloc(&p.hi, nhi * sizeof(Fr)) != cudaSuccess ||
-      cudaMemcpy(p.lo, lo.data(), nlo * sizeof(Fr), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(p.hi, hi.data(), nhi * sizeof(Fr), cudaMemcpyHostToDevice) != cudaSuccess) {
-    if (p.lo) cudaFree(p.lo);
-    if (p.hi) cudaFree(p.hi);
-    return nullptr;
+  Fr* t = nullptr;
+  if (logn <= 11) {
+    if (upload(&t, pow_table(gen, size_t(1) << logn))) return nullptr;
+  } else {
+    const int lc = (logn + 1) / 2, lr = logn - lc;
+    Fr *lo = nullptr, *hi = nullptr;
+    int rc = upload(&lo, pow_table(gen, size_t(1) << lc));
+    if (!rc) rc = upload(&hi, pow_table(gen.pow_u64(uint64_t(1) << lc), size_t(1) << lr));
+    if (!rc) rc = build_full_table(lo, hi, lr, lc, true, Fr::one(), &t);
+    if (lo) cudaFree(lo);
+    if (hi) cudaFree(hi);
+    if (rc) return nullptr;
   }
-  return &(g_coset_pows[key] = p);
+  return g_coset_pows[key] = t;
+}
+
+// the column pass's factors of a transform of zg_ntt (with 1/N for the
+// inverse), one direction at a time; null on failure
+const Fr* cached_full_twiddles(const Twiddles* tw, bool inverse) {
+  std::lock_guard<std::mutex> g(g_ntt_mu);
+  Twiddles* t = const_cast<Twiddles*>(tw);  // an entry of g_ntt_tw
+  Fr** full = inverse ? &t->wni_full : &t->wn_full;
+  if (!*full) {
+    const Fr ninv = host_fr_from_u32(1u << (tw->lr + tw->lc)).inverse();
+    if (build_full_table(inverse ? tw->wni_lo : tw->wn_lo, inverse ? tw->wni_hi : tw->wn_hi, tw->lr, tw->lc, false,
+                         inverse ? ninv : Fr::one(), full))
+      return nullptr;
+  }
+  return *full;
 }
 
 // The stream-ordered pool of the current device keeps freed memory instead of
@@ -3418,34 +3454,35 @@ int zg_ntt(void* d_data, uint32_t log_n, uint32_t batch, int inverse, uint32_t c
   ZG_CK(cudaFuncSetAttribute(k_ntt_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   const size_t n = size_t(1) << log_n;
   Fr* v = (Fr*)d_data;
-  const CosetPows* cp = nullptr;
-  if (coset_idx && !(cp = cached_coset_pows((int)log_n, coset_idx))) return fail(ZG_ERR_CUDA, "coset table alloc failed");
-  const Fr ninv = host_fr_from_u32((uint32_t)n).inverse();
+  const Fr* cs = nullptr;
+  if (coset_idx && !(cs = cached_coset_pows((int)log_n, coset_idx))) return fail(ZG_ERR_CUDA, "coset table alloc failed");
   // the transforms run on the canonical values directly (linear passes with
   // Montgomery-form twiddles keep canonical values canonical); the coset
-  // shift and the inverse's 1/n are products in the transforms' first loads
-  // and last stores
+  // shift is a product of the transforms' first loads, the inverse's 1/n part
+  // of the last stores' or of the column pass's factors
   if (log_n <= 11) {
     const Twiddles* tw = cached_twiddles(0, (int)log_n);
     if (!tw) return ZG_ERR_CUDA;
+    const Fr ninv = inverse ? host_fr_from_u32((uint32_t)n).inverse() : Fr::one();
     for (uint32_t b0 = 0; b0 < batch;) {
       uint32_t nb = std::min<uint32_t>(batch - b0, 65535);
       k_ntt_small<<<nb, ntt_threads((int)log_n), n * sizeof(Fr), s>>>(
-          v + (size_t)b0 * n, (int)log_n, inverse ? tw->twi_c : tw->twf_c, cp ? cp->lo : nullptr, inverse, ninv);
+          v + (size_t)b0 * n, (int)log_n, inverse ? tw->twi_c : tw->twf_c, cs, inverse, ninv);
       b0 += nb;
     }
   } else {
     const int lc = (int)(log_n + 1) / 2, lr = (int)log_n - lc;
     const Twiddles* tw = cached_twiddles(lr, lc);
     if (!tw) return ZG_ERR_CUDA;
+    const Fr* wfull = cached_full_twiddles(tw, inverse != 0);
+    if (!wfull) return ZG_ERR_CUDA;
     const uint32_t per = std::min<uint32_t>(batch, 65535);
     keep_pool_memory();
     Fr* tmp = nullptr;
     ZG_CK(cudaMallocAsync(&tmp, (size_t)per * n * sizeof(Fr), s));
     for (uint32_t b0 = 0; b0 < batch; b0 += per) {
       const uint32_t nb = std::min<uint32_t>(batch - b0, per);
-      ntt4(*tw, v + (size_t)b0 * n, tmp, v + (size_t)b0 * n, inverse != 0, s, nb, cp ? cp->lo : nullptr,
-           cp ? cp->hi : nullptr, cp ? cp->h : 0, inverse ? &ninv : nullptr);
+      ntt4(*tw, v + (size_t)b0 * n, tmp, v + (size_t)b0 * n, inverse != 0, s, nb, wfull, cs);
     }
     cudaFreeAsync(tmp, s);
   }

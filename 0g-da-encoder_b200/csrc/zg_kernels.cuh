@@ -1415,15 +1415,31 @@ __global__ void k_quot_coeff(const Fr* pw, Fr* c, uint32_t M, uint32_t n) {
   c[i] = (i >= 1 && i <= M) ? pw[M - i] : Fr::zero();
 }
 
+// out[s R + r] = base^(s r) scale (shift 0) or base^(r C + s) scale, with lo[i] =
+// base^i (i < C) and hi[i] = base^(C i) (i < R)
+__global__ void __launch_bounds__(256) k_full_table(const Fr* __restrict__ lo, const Fr* __restrict__ hi, int lr, int lc,
+                                                    int shift, Fr scale, Fr* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, nmask = (1u << (lr + lc)) - 1;
+  if (i > nmask) return;
+  const uint32_t s = i >> lr, r = i & ((1u << lr) - 1);
+  out[i] = pow_split(lo, hi, shift ? (r << lc) + s : s * r, lc, nmask) * scale;
+}
+
 // generic four-step NTT pass A: for each column s (C of them) of x viewed as
 // [R][C] row-major: R-point transform over q, times w_N^{s r}; writes Y[r][s].
 // blockIdx.y selects the vector of a batch (vectors of R C elements back to back).
-// With cs_lo set, element i of x is first multiplied by
-// cs_lo[i mod 2^cs_h] * cs_hi[i >> cs_h] (the coset shift).
+// With cs set, element q C + s of x is first multiplied by cs[s R + q] (the
+// coset shift); with wfull set the factors w_N^{s r} (and a scale) are
+// wfull[s R + r], read in order by the CTA of column s, else products of the
+// split tables. Bound by the field products (N (log2 N) / 2 of them and one per
+// factor); the full tables take two products per element of a coset transform
+// away (the power w_N^{s r} and the coset's lo hi) and the 1/N product of the
+// last stores: 64 coset transforms of 2^14 207 -> 159 us, one inverse of 2^20
+// 247 -> 209 us, 20% and 33% above the products' own time.
 __global__ void __launch_bounds__(256) k_ntt4_colpass(const Fr* __restrict__ x, Fr* __restrict__ y, int lr, int lc,
                                const Fr* __restrict__ tw_r, const Fr* __restrict__ w_lo,
-                               const Fr* __restrict__ w_hi, const Fr* __restrict__ cs_lo,
-                               const Fr* __restrict__ cs_hi, int cs_h) {
+                               const Fr* __restrict__ w_hi, const Fr* __restrict__ wfull,
+                               const Fr* __restrict__ cs) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int C = 1 << lc;
   Fr* s = reinterpret_cast<Fr*>(smem);
@@ -1432,18 +1448,18 @@ __global__ void __launch_bounds__(256) k_ntt4_colpass(const Fr* __restrict__ x, 
   y += (size_t)blockIdx.y << (lr + lc);
   const uint32_t nmask = (1u << (lr + lc)) - 1;
   auto get = [&](int q) {
-    const uint32_t i = (uint32_t)q * C + col;
-    const Fr e = load_fr(x + i);
-    return cs_lo ? e * (cs_lo[i & ((1u << cs_h) - 1)] * cs_hi[i >> cs_h]) : e;
+    const Fr e = load_fr(x + (size_t)q * C + col);
+    return cs ? e * load_fr(cs + ((size_t)col << lr) + q) : e;
   };
   ntt_block(s, lr, tw_r, get, [&](int r, const Fr& v) { s[r] = v; });
-  for (int r = threadIdx.x; r < (1 << lr); r += blockDim.x)
-    store_fr(y + (size_t)r * C + col, s[r] * pow_split(w_lo, w_hi, col * (uint32_t)r, lc, nmask));
+  for (int r = threadIdx.x; r < (1 << lr); r += blockDim.x) {
+    const Fr w = wfull ? load_fr(wfull + ((size_t)col << lr) + r) : pow_split(w_lo, w_hi, col * (uint32_t)r, lc, nmask);
+    store_fr(y + (size_t)r * C + col, s[r] * w);
+  }
 }
 // pass B: for each r, C-point transform over s of Y[r][*]; out[j R + r]
-// (times scale when do_scale)
 __global__ void __launch_bounds__(256) k_ntt4_rowpass(const Fr* __restrict__ y, Fr* __restrict__ out, int lr, int lc,
-                               const Fr* __restrict__ tw_c, int do_scale, Fr scale) {
+                               const Fr* __restrict__ tw_c) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int R = 1 << lr, C = 1 << lc;
   Fr* s = reinterpret_cast<Fr*>(smem);
@@ -1451,7 +1467,7 @@ __global__ void __launch_bounds__(256) k_ntt4_rowpass(const Fr* __restrict__ y, 
   y += (size_t)blockIdx.y << (lr + lc);
   out += (size_t)blockIdx.y << (lr + lc);
   ntt_block(s, lc, tw_c, [&](int k) { return load_fr(y + (size_t)r * C + k); },
-            [&](int j, const Fr& v) { store_fr(out + (size_t)j * R + r, do_scale ? v * scale : v); });
+            [&](int j, const Fr& v) { store_fr(out + (size_t)j * R + r, v); });
 }
 
 // fixed-base table of G: tab[w*255 + d - 1] = d * 2^{8w} * G (XYZZ)
