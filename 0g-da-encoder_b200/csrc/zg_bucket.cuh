@@ -152,8 +152,30 @@ static __device__ __noinline__ AffCase aff_case(const G1Aff a, const G1Aff b) {
   return r;
 }
 
+#ifdef __CUDACC__
+__device__ __forceinline__ Fq fq_lane_xor(const Fq& x, int d) {
+  Fq r;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r.v[i] = __shfl_xor_sync(0xffffffffu, x.v[i], d);
+  return r;
+}
+// the inverse of each lane's c (a whole warp calls): one inversion per quad of
+// the four lanes' product, four products in a row more
+template <class M>
+__device__ __forceinline__ Fq warp_inverse(const Fq& c) {
+  const Fq c1 = fq_lane_xor(c, 1), p = M::mul(c, c1), p2 = fq_lane_xor(p, 2);
+  return M::mul(M::mul(Fq::inverse_quad(M::mul(p, p2)), p2), c1);
+}
+#else
+template <class M>
+Fq warp_inverse(const Fq& c) {
+  return c.inverse();
+}
+#endif
+
 // Inverts every thread's v (nonzero): the threads' values are multiplied into
-// 32 products that one warp inverts lane by lane, `turn` picking the warp.
+// 32 products that one warp inverts, `turn` picking the warp. Where a launch
+// has few items, these inversions are its time.
 template <class M>
 __device__ __forceinline__ Fq block_inverse(const Fq& v, Fq* sp, uint32_t turn) {
   constexpr int N = FB_ACC_THREADS / 32;
@@ -165,7 +187,7 @@ __device__ __forceinline__ Fq block_inverse(const Fq& v, Fq* sp, uint32_t turn) 
     c[0] = sp[lane];
 #pragma unroll
     for (int i = 1; i < N; ++i) c[i] = M::mul(c[i - 1], sp[lane + 32 * i]);
-    Fq inv = c[N - 1].inverse();
+    Fq inv = warp_inverse<M>(c[N - 1]);
 #pragma unroll
     for (int i = N - 1; i >= 1; --i) {
       const Fq x = sp[lane + 32 * i];

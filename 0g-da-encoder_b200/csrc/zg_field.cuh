@@ -33,9 +33,9 @@ struct FqCfg {
                             r2_4 = 0x0a417ff6u, r2_5 = 0x47ab1effu, r2_6 = 0xcab8351fu, r2_7 = 0x06d89f71u;
   static constexpr uint32_t one0 = 0xc58f0d9du, one1 = 0xd35d438du, one2 = 0xf5c70b3du, one3 = 0x0a78eb28u,
                             one4 = 0x7879462cu, one5 = 0x666ea36fu, one6 = 0x9a07df2fu, one7 = 0x0e0a77c1u;
-  // 2^(40 + 512) mod p, the start of inverse()
-  static constexpr uint32_t gcd0 = 0x16fe05fbu, gcd1 = 0xda94bc1bu, gcd2 = 0x51de3187u, gcd3 = 0xfdb7603bu,
-                            gcd4 = 0xe1594d7eu, gcd5 = 0x5dbd35a2u, gcd6 = 0x9d0994cdu, gcd7 = 0x16579a57u;
+  // 2^(30 + 512) mod p, the start of inverse()
+  static constexpr uint32_t gcd0 = 0xe0d1e109u, gcd1 = 0x54964889u, gcd2 = 0x580bb0b7u, gcd3 = 0xf5c72b3bu,
+                            gcd4 = 0xf3b7923cu, gcd5 = 0x9507f0f3u, gcd6 = 0x65a80820u, gcd7 = 0x03f1b742u;
 };
 struct FrCfg {
   static constexpr uint32_t p0 = 0xf0000001u, p1 = 0x43e1f593u, p2 = 0x79b97091u, p3 = 0x2833e848u,
@@ -45,8 +45,8 @@ struct FrCfg {
                             r2_4 = 0x53bb8085u, r2_5 = 0x8c49833du, r2_6 = 0x7f4e44a5u, r2_7 = 0x0216d0b1u;
   static constexpr uint32_t one0 = 0x4ffffffbu, one1 = 0xac96341cu, one2 = 0x9f60cd29u, one3 = 0x36fc7695u,
                             one4 = 0x7879462eu, one5 = 0x666ea36fu, one6 = 0x9a07df2fu, one7 = 0x0e0a77c1u;
-  static constexpr uint32_t gcd0 = 0x82bf4ec7u, gcd1 = 0x9126b014u, gcd2 = 0xf84ec615u, gcd3 = 0x89ec5f7du,
-                            gcd4 = 0x2dc5f176u, gcd5 = 0xeeab1253u, gcd6 = 0xc17c9526u, gcd7 = 0x0e680cefu;
+  static constexpr uint32_t gcd0 = 0x7d3cafd4u, gcd1 = 0xec641afcu, gcd2 = 0x06b30259u, gcd3 = 0xd72c58d8u,
+                            gcd4 = 0x9de13abeu, gcd5 = 0x0a523413u, gcd6 = 0xd945ca5au, gcd7 = 0x0ece42fdu;
 };
 
 template <class C>
@@ -390,66 +390,198 @@ struct Fp {
   // inversion", TCHES 2019, with the half-integer delta that needs at most 590
   // steps for 256-bit operands), run 30 at a time on the low words of f and g;
   // each batch of 30 is a 2 x 2 matrix of 31-bit entries that is applied to
-  // f, g (signed 30-bit limbs, an exact division by 2^30) and to d, e (mod p,
-  // f = d x 2^(2k) and g = e x 2^(2k) mod p after k batches: every batch
-  // divides d and e by 2^32 in one Montgomery row). 20 batches end with
-  // f = +-1, g = 0, so the inverse is +-d for the start e = 2^40 R^2. A lone
-  // warp takes 21 us on a B200, against 165 us for the exponentiation by p - 2
-  // (380 products in a row).
+  // f, g (signed 30-bit limbs, an exact division by 2^30) and to d, e (the same
+  // limbs; a multiple of p makes the division exact). d a = f S and e a = g S
+  // mod p hold throughout for the start e = S; 20 batches end with f = +-1,
+  // g = 0, so d = +-S / a, and a last division by 2^30 brings |d| <= 11 p
+  // (each batch adds up to p / 2) below p.
+  // A lone warp's time is the instructions of the 600 steps. x and the matrix'
+  // first row double instead of y halving (bit k of y is tested in step k), a
+  // row's two entries share a word (15 steps keep them in 16 bits each): 12
+  // instructions a step. A lone warp takes 36 000 cycles on a B200 (40 000
+  // with two words a row, y halving and 32-bit limbs of d and e), against some
+  // 310 000 for the exponentiation by p - 2 (380 products in a row).
   ZG_HD Fp inverse() const {
-    constexpr int32_t M30 = (1 << 30) - 1;
-    int32_t f[9], g[9];
-    const Fp p = modulus();
-    limbs30(p, f);
+    int32_t f[9], g[9], d[9], e[9];
+    limbs30(modulus(), f);
     limbs30(*this, g);
-    Fp d = zero(), e;
-    e.v[0] = C::gcd0; e.v[1] = C::gcd1; e.v[2] = C::gcd2; e.v[3] = C::gcd3;
-    e.v[4] = C::gcd4; e.v[5] = C::gcd5; e.v[6] = C::gcd6; e.v[7] = C::gcd7;
-    int32_t delta2 = 1;  // 2 delta
+    limbs30(gcd_start(), e);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) d[i] = 0;
+    int32_t nd2 = -1;  // -2 delta
 #pragma unroll 1
     for (int batch = 0; batch < 20; ++batch) {
-      // rows (u, v) and (q, r): 2^30 f' = u f + v g, 2^30 g' = q f + r g
-      int32_t u = 1, v = 0, q = 0, r = 1;
       uint32_t x = (uint32_t)f[0] | (uint32_t)f[1] << 30, y = (uint32_t)g[0] | (uint32_t)g[1] << 30;
-#pragma unroll 6
-      for (int k = 0; k < 30; ++k) {
-        const bool odd = (y & 1u) != 0, swap = odd && delta2 > 0;
-        const uint32_t ax = odd ? (swap ? 0u - x : x) : 0u;
-        const int32_t au = odd ? (swap ? -u : u) : 0, av = odd ? (swap ? -v : v) : 0;
-        if (swap) {
-          x = y;
-          u = q;
-          v = r;
-          delta2 = -delta2;
-        }
-        delta2 += 2;
-        y = (y + ax) >> 1;
-        q += au;
-        r += av;
-        u *= 2;
-        v *= 2;
-      }
-      const Fp nd = raw_neg(d), ne = raw_neg(e);
-      const Fp d1 = gcd_row(u < 0 ? nd : d, v < 0 ? ne : e, u, v);
-      e = gcd_row(q < 0 ? nd : d, r < 0 ? ne : e, q, r);
-      d = d1;
-      int64_t cf = (int64_t)u * f[0] + (int64_t)v * g[0];
-      int64_t cg = (int64_t)q * f[0] + (int64_t)r * g[0];
-      cf >>= 30;
-      cg >>= 30;
-#pragma unroll
-      for (int i = 1; i < 9; ++i) {
-        cf += (int64_t)u * f[i] + (int64_t)v * g[i];
-        cg += (int64_t)q * f[i] + (int64_t)r * g[i];
-        f[i - 1] = (int32_t)cf & M30;
-        g[i - 1] = (int32_t)cg & M30;
-        cf >>= 30;
-        cg >>= 30;
-      }
-      f[8] = (int32_t)cf;
-      g[8] = (int32_t)cg;
+      int32_t u1, v1, q1, r1, u2, v2, q2, r2;
+      gcd_steps<0>(x, y, nd2, u1, v1, q1, r1);
+      gcd_steps<15>(x, y, nd2, u2, v2, q2, r2);
+      const int32_t u = u2 * u1 + v2 * q1, v = u2 * v1 + v2 * r1;
+      const int32_t q = q2 * u1 + r2 * q1, r = q2 * v1 + r2 * r1;
+      gcd_rows<false>(f, g, u, v, q, r);
+      gcd_rows<true>(d, e, u, v, q, r);
     }
-    return f[8] < 0 ? neg(d) : d;
+    // d / 2^30, with the sign of f
+    gcd_rows<true>(d, e, f[8] < 0 ? -1 : 1, 0, 0, 0);
+    return from_limbs30(d);
+  }
+#ifdef __CUDACC__
+  // inverse() with the four lanes of a quad (a whole warp calls; a is the same
+  // in all four, and so is the result): each lane has the batch's division
+  // steps and one column of its matrix, then one of the rows f, g, d, e, whose
+  // limbs it exchanges with its neighbour. 26 800 cycles of a lone warp.
+  static __device__ __noinline__ Fp inverse_quad(const Fp a) {
+    constexpr int32_t M30 = (1 << 30) - 1;
+    const uint32_t all = 0xffffffffu, quad = threadIdx.x & 28u, row = threadIdx.x & 3u;
+    const bool odd = row & 1u;
+    int32_t m[9], p[9];
+    {
+      const Fp mod = modulus(), start = gcd_start();
+      Fp x;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x.v[i] = row == 0 ? mod.v[i] : row == 1 ? a.v[i] : row == 2 ? 0u : start.v[i];
+      limbs30(x, m);
+      limbs30(mod, p);
+    }
+    int32_t nd2 = -1;
+#pragma unroll 1
+    for (int batch = 0; batch <= 20; ++batch) {
+      int32_t own, other;  // this row' = own this row + other the neighbour's
+      if (batch < 20) {
+        const uint32_t w = (uint32_t)m[0] | (uint32_t)m[1] << 30;
+        uint32_t x = __shfl_sync(all, w, quad), y = __shfl_sync(all, w, quad + 1);
+        uint32_t U = odd ? 0u : 1u, Q = odd ? 1u : 0u;
+#pragma unroll
+        for (int k = 0; k < 30; ++k) {
+          gcd_step(x, y, U, Q, nd2, k);
+          U <<= 1;
+        }
+        own = (int32_t)(odd ? Q : U);
+        other = (int32_t)__shfl_xor_sync(all, odd ? U : Q, 1);
+      } else {  // the division by 2^30 that ends inverse(), with the sign of f
+        own = (int32_t)__shfl_sync(all, (uint32_t)m[8], quad) < 0 ? -1 : 1;
+        other = 0;
+      }
+      int64_t c = 0;
+      int32_t k = 0;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const int32_t n = (int32_t)__shfl_xor_sync(all, (uint32_t)m[i], 1);
+        c += (int64_t)own * m[i] + (int64_t)other * n;
+        if (i == 0 && row >= 2) k = (int32_t)((uint32_t)c * C::inv << 2) >> 2;
+        c += (int64_t)k * p[i];
+        if (i) m[i - 1] = (int32_t)c & M30;
+        c >>= 30;
+      }
+      m[8] = (int32_t)c;
+    }
+    Fp r = from_limbs30(m);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r.v[i] = __shfl_sync(all, r.v[i], quad + 2);
+    return r;
+  }
+#endif
+  ZG_HD static Fp gcd_start() {
+    Fp r;
+    r.v[0] = C::gcd0; r.v[1] = C::gcd1; r.v[2] = C::gcd2; r.v[3] = C::gcd3;
+    r.v[4] = C::gcd4; r.v[5] = C::gcd5; r.v[6] = C::gcd6; r.v[7] = C::gcd7;
+    return r;
+  }
+  // 15 division steps, K done before them on these words: x and y are 2^K times
+  // their values (mod 2^32). (u, v) and (q, r) receive the rows of
+  // 2^15 f' = u f + v g, 2^15 g' = q f + r g. The first row is kept undoubled by
+  // the last step, so |u|, |v| <= 2^14 fit their half words; |q| + |r| <= 2^15,
+  // and neither is 2^15 alone (u and v are even, the determinant is 2^15).
+  template <int K>
+  ZG_HD static void gcd_steps(uint32_t& x, uint32_t& y, int32_t& nd2, int32_t& u, int32_t& v, int32_t& q, int32_t& r) {
+    uint32_t U = 1u, Q = 1u << 16;
+#pragma unroll
+    for (int k = K; k < K + 15; ++k) {
+      gcd_step(x, y, U, Q, nd2, k);
+      if (k < K + 14) U <<= 1;
+    }
+    u = (int16_t)U;
+    v = (int32_t)(U - (uint32_t)u) >> 16;
+    q = (int16_t)Q;
+    r = (int32_t)(Q - (uint32_t)q) >> 16;
+    u *= 2;
+    v *= 2;
+  }
+  // one division step on bit k of y: (x, y) and, alike, the matrix rows (U, Q);
+  // nd2 = -2 delta. Predicated: what a lone warp waits for is the chain of
+  // instructions from one tested bit to the next.
+  ZG_HD static void gcd_step(uint32_t& x, uint32_t& y, uint32_t& U, uint32_t& Q, int32_t& nd2, int k) {
+#ifdef __CUDA_ARCH__
+    asm("{\n\t.reg .pred o, s, n;\n\t.reg .b32 t;\n\t"
+        "and.b32 t, %1, %5;\n\t"
+        "setp.ne.u32 o, t, 0;\n\t"
+        "setp.lt.and.s32 s|n, %4, 0, o;\n\t"
+        "@s sub.u32 %1, %1, %0;\n\t"
+        "@n add.u32 %1, %1, %0;\n\t"
+        "@s neg.s32 %4, %4;\n\t"
+        "@s sub.u32 %3, %3, %2;\n\t"
+        "@n add.u32 %3, %3, %2;\n\t"
+        "@s add.u32 %0, %0, %1;\n\t"
+        "@s add.u32 %2, %2, %3;\n\t"
+        "add.s32 %4, %4, -2;\n\t"
+        "shl.b32 %0, %0, 1;\n\t}"
+        : "+r"(x), "+r"(y), "+r"(U), "+r"(Q), "+r"(nd2)
+        : "r"(1u << k));
+#else
+    const bool odd = (y >> k & 1u) != 0, swap = odd && nd2 < 0;
+    if (odd) {
+      y = swap ? y - x : y + x;
+      Q = swap ? Q - U : Q + U;
+    }
+    if (swap) {  // x = the old y
+      x += y;
+      U += Q;
+      nd2 = -nd2;
+    }
+    nd2 -= 2;
+    x <<= 1;
+#endif
+  }
+  // a, b = (u a + v b) / 2^30, (q a + r b) / 2^30 in signed 30-bit limbs (limbs 0
+  // to 7 in [0, 2^30)), mod p (a multiple of p below 2^29 p makes the division
+  // exact) or exact already
+  template <bool MOD>
+  ZG_HD static void gcd_rows(int32_t* a, int32_t* b, int32_t u, int32_t v, int32_t q, int32_t r) {
+    constexpr int32_t M30 = (1 << 30) - 1;
+    int32_t p[9], ka = 0, kb = 0;
+    limbs30(modulus(), p);
+    int64_t ca = (int64_t)u * a[0] + (int64_t)v * b[0], cb = (int64_t)q * a[0] + (int64_t)r * b[0];
+    if (MOD) {
+      ka = (int32_t)((uint32_t)ca * C::inv << 2) >> 2;
+      kb = (int32_t)((uint32_t)cb * C::inv << 2) >> 2;
+      ca += (int64_t)ka * p[0];
+      cb += (int64_t)kb * p[0];
+    }
+    ca >>= 30;
+    cb >>= 30;
+#pragma unroll
+    for (int i = 1; i < 9; ++i) {
+      ca += (int64_t)u * a[i] + (int64_t)v * b[i];
+      cb += (int64_t)q * a[i] + (int64_t)r * b[i];
+      if (MOD) {
+        ca += (int64_t)ka * p[i];
+        cb += (int64_t)kb * p[i];
+      }
+      a[i - 1] = (int32_t)ca & M30;
+      b[i - 1] = (int32_t)cb & M30;
+      ca >>= 30;
+      cb >>= 30;
+    }
+    a[8] = (int32_t)ca;
+    b[8] = (int32_t)cb;
+  }
+  // signed 30-bit limbs of a value below 2^256 in absolute terms, p added if
+  // it is negative
+  ZG_HD static Fp from_limbs30(const int32_t* l) {
+    Fp t, s;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t.v[i] = (uint32_t)l[i] >> (2 * i) | (uint32_t)l[i + 1] << (30 - 2 * i);
+    add_raw(s, t, modulus());
+    return l[8] < 0 ? s : t;
   }
   ZG_HD static void limbs30(const Fp& a, int32_t* l) {
 #pragma unroll
@@ -459,32 +591,6 @@ struct Fp {
       if (s > 2 && w + 1 < 8) x |= a.v[w + 1] << (32 - s);
       l[i] = (int32_t)(x & ((1u << 30) - 1));
     }
-  }
-  ZG_HD static Fp raw_neg(const Fp& a) {  // p - a for a <= p, not reduced
-    Fp r;
-    sub_raw(r, modulus(), a);
-    return r;
-  }
-  // (|u| a + |v| b) / 2^32 mod p for a, b <= p and |u| + |v| <= 2^30
-  ZG_HD static Fp gcd_row(const Fp& a, const Fp& b, int32_t u, int32_t v) {
-    const uint32_t au = (uint32_t)(u < 0 ? -u : u), av = (uint32_t)(v < 0 ? -v : v);
-    const Fp p = modulus();
-    uint64_t s = (uint64_t)a.v[0] * au + (uint64_t)b.v[0] * av;
-    const uint32_t k = (uint32_t)s * C::inv;
-    // the low word cancels: its sum with k p_0's is 0 or 2^32
-    uint64_t carry = (s >> 32) + (((uint64_t)k * p.v[0]) >> 32) + ((uint32_t)s != 0 ? 1u : 0u);
-    Fp t;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) {
-      s = (uint64_t)a.v[i] * au + (uint64_t)b.v[i] * av + carry;
-      const uint64_t w = (uint64_t)k * p.v[i] + (uint32_t)s;
-      t.v[i - 1] = (uint32_t)w;
-      carry = (s >> 32) + (w >> 32);
-    }
-    t.v[7] = (uint32_t)carry;
-    Fp red;
-    const uint32_t borrow = sub_raw(red, t, p);
-    return borrow ? t : red;
   }
   // canonical value > (p-1)/2, i.e. ark's "y > -y" (SWFlags::YIsNegative)
   ZG_HD bool canonical_is_negative() const {
