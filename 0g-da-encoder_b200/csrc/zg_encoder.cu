@@ -197,11 +197,7 @@ int set_smem_limits() {
   ZG_CK(cudaFuncSetAttribute(k_rows_ntt, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_msm_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_fb_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_wd_sort<15>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_wd_sort<14>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_wd_sort<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_wd_sort<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_wd_sort<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  ZG_CK(cudaFuncSetAttribute(k_wd_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_ntt4_colpass, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_ntt4_rowpass, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   done.insert(dev);
@@ -261,8 +257,8 @@ struct Lane {
   int cap = 0;                  // blob slots
   Fr* T1 = nullptr;             // [R][C] row-iNTT output
   Fr* Bc = nullptr;             // [2][R][C] column-pass output
-  uint32_t* fb_offs = nullptr;  // [cap][3R][FB_BUCKETS + 1]
-  uint16_t* fb_ents = nullptr;  // [cap][3R][FB_WINDOWS C]
+  uint32_t* fb_offs = nullptr;  // [cap][chunk_offs]
+  uint16_t* fb_ents = nullptr;  // [cap][chunk_ents]
   struct Wd {
     uint32_t* offs = nullptr;   // [cap][3][units][2^ulog + 1]
     uint32_t* ents = nullptr;   // [cap][3][units][W 2^ulog]
@@ -303,7 +299,7 @@ struct zg_ctx {
   // mlog = 1 its items merge pairs of sort units (units of 2^(ulog + 1)
   // points sharing 2^ulog buckets), and the class reads the sort output of
   // class sort_of (the first class of the same ulog, which runs the sort).
-  // The 11-bit chunk items cover the other lines, n_l0 .. n_l0 + n_lines - 1.
+  // The 11-bit items (chunk_sets) cover the other lines, n_l0 .. n_l0 + n_lines - 1.
   struct WdClass {
     int ulog = 0, mlog = 0, sort_of = 0, W = 0, l0 = 0, nl = 0, hi_last = 0;
     G1Aff* tab = nullptr;
@@ -532,21 +528,76 @@ void apply_wide_classes(zg_ctx* c, int on) {
   c->n_lines = c->lr + 1 - next + (high ? 0 : 1);
 }
 
-// work items of one blob's MSM: every (coset, chunk or unit block, line),
-// the chunk lines first, then each wide class in use (a merged class has half
+// The 11-bit items of one blob's MSM as sets of table lines l0 .. l0 + nl - 1
+// whose items take units of 2^ulog points. With 2^FB_UNIT_LOG columns or more
+// the units are the chunks (2^lc points). With fewer, an item's fixed costs
+// (the 2048 additions of its bucket grid, its combine) outweigh its entries,
+// so a line whose nodes span several chunks takes them together, up to
+// 2^FB_UNIT_LOG points and no more than its nodes hold (2^(lr + lc - 1 - l)
+// for quotient line l, 2^lc for the basis line, whose sums over the chunks are
+// results themselves, 2^(lr + lc) for the high line): 960 items instead of
+// 1536 for 64 x 32. That blob took 1665 us with chunks alone, 1509 with units
+// of 64 points, 1588 with 128 and 1920 with 256, whose items are too uneven
+// for the few CTAs they fill.
+constexpr int FB_UNIT_LOG = 6;
+struct ChunkSet {
+  int ulog, l0, nl;
+};
+struct ChunkSets {
+  int n = 0;
+  ChunkSet s[FB_MAX_CHUNK_SETS];
+};
+ChunkSets chunk_sets(const zg_ctx* c) {
+  ChunkSets r;
+  if (c->lc >= FB_UNIT_LOG) {
+    r.s[r.n++] = ChunkSet{c->lc, c->n_l0, c->n_lines};
+    return r;
+  }
+  const int top = std::min(FB_UNIT_LOG, c->lc + FB_MAX_CHUNK_SETS - 2);
+  for (int l = 0; l <= c->lr; ++l) {
+    const int u = l < c->lr ? std::min(top, c->lr + c->lc - 1 - l) : c->lc;
+    if (r.n && r.s[r.n - 1].ulog == u) ++r.s[r.n - 1].nl;
+    else r.s[r.n++] = ChunkSet{u, l, 1};
+  }
+  r.s[r.n++] = ChunkSet{std::min(top, c->lr + c->lc), c->L - 1, 1};
+  return r;
+}
+uint32_t chunk_set_items(const zg_ctx* c, const ChunkSet& cs) { return (uint32_t)(3 * (c->N >> cs.ulog) * cs.nl); }
+// units that a blob's chunk sets sort, and where set k's begin
+uint32_t chunk_units(const zg_ctx* c, const ChunkSets& cs, int k) {
+  uint32_t u = 0;
+  for (int j = 0; j < k; ++j) u += (uint32_t)(3 * (c->N >> cs.s[j].ulog));
+  return u;
+}
+
+// work items of one blob's MSM: every (coset, unit or unit block, line), the
+// chunk sets first, then each wide class in use (a merged class has half
 // the items per line); blob_items_max bounds it for every choice of classes
 uint32_t blob_items_max(const zg_ctx* c) { return (uint32_t)(3 * c->R * c->L); }
+uint32_t blob_chunk_items(const zg_ctx* c) {
+  const ChunkSets cs = chunk_sets(c);
+  uint32_t u = 0;
+  for (int k = 0; k < cs.n; ++k) u += chunk_set_items(c, cs.s[k]);
+  return u;
+}
 uint32_t blob_items(const zg_ctx* c) {
-  uint32_t u = (uint32_t)(3 * c->R * c->n_lines);
+  uint32_t u = blob_chunk_items(c);
   for (int j = 0; j < c->wd_on; ++j) u += (uint32_t)(3 * (c->R >> c->wd[j].mlog) * c->wd[j].nl);
   return u;
 }
+// sizes of a blob's sort output: offsets of every unit, entries of every set
+// (never less than the R chunks per coset of the single MSMs)
+size_t chunk_offs(const zg_ctx* c) {
+  const ChunkSets cs = chunk_sets(c);
+  return (size_t)std::max<uint64_t>(chunk_units(c, cs, cs.n), 3 * c->R) * (FB_BUCKETS + 1);
+}
+size_t chunk_ents(const zg_ctx* c) { return (size_t)chunk_sets(c).n * 3 * c->N * FB_WINDOWS; }
 
 // k_fb_accum's segment size: the entries of FB_GROUP of a context's largest
 // items, a wide unit's block 0 counted with half as many again, within
 // FB_CAP_MAX
 uint32_t fb_segment(const zg_ctx* c) {
-  uint32_t n = (uint32_t)(FB_WINDOWS * c->C);
+  uint32_t n = (uint32_t)FB_WINDOWS << std::max(c->lc, FB_UNIT_LOG);
   for (const zg_ctx::WdClass& k : c->wd) n = std::max(n, ((uint32_t)wd_windows(k.ulog) * 1536u) << k.mlog);
   return std::min((uint32_t)FB_GROUP * n, FB_CAP_MAX);
 }
@@ -558,7 +609,7 @@ size_t lane_bytes(const zg_ctx* c, int cap) {
   size_t b = 3 * N * sizeof(Fr);
   size_t per = 3 * (size_t)c->L * R * sizeof(XYZZ) + 3 * (4 * R - 2) * sizeof(XYZZ);
   if (c->fb) {
-    per += 3 * R * (FB_BUCKETS + 1) * 4 + 3 * R * FB_WINDOWS * c->C * 2 +
+    per += chunk_offs(c) * 4 + chunk_ents(c) * 2 +
            (size_t)blob_items_max(c) * FB_OUT * sizeof(G1Aff);
     for (size_t j = 0; j < c->wd.size(); ++j) {
       const zg_ctx::WdClass& k = c->wd[j];
@@ -591,8 +642,8 @@ int alloc_lane(zg_ctx* c, Lane* ln, int cap) {
   ZG_CK(cudaMalloc(&ln->T1, N * sizeof(Fr)));
   ZG_CK(cudaMalloc(&ln->Bc, 2 * N * sizeof(Fr)));
   if (c->fb) {
-    ZG_CK(cudaMalloc(&ln->fb_offs, k * 3 * R * (FB_BUCKETS + 1) * sizeof(uint32_t)));
-    ZG_CK(cudaMalloc(&ln->fb_ents, k * 3 * R * FB_WINDOWS * c->C * sizeof(uint16_t)));
+    ZG_CK(cudaMalloc(&ln->fb_offs, k * chunk_offs(c) * sizeof(uint32_t)));
+    ZG_CK(cudaMalloc(&ln->fb_ents, k * chunk_ents(c) * sizeof(uint16_t)));
     ZG_CK(cudaMalloc(&ln->fb_out, k * blob_items_max(c) * FB_OUT * sizeof(G1Aff)));
     ln->wd.resize(c->wd.size());
     for (size_t j = 0; j < c->wd.size(); ++j) {
@@ -860,35 +911,61 @@ BlobBufs ctx_bufs(zg_ctx* c) {
 uint64_t launches_per_encode(const zg_ctx* c, int nb = 1) {
   uint64_t merkle = 0;
   merkle_plan(c->tree_depth, [&](int, int, int) { ++merkle; });
-  uint64_t sorts = 0;  // the wide classes in use that run their own digit sort
-  for (int k = 0; k < c->wd_on; ++k) sorts += c->wd[k].sort_of == k ? 1 : 0;
+  const uint64_t sorts = c->wd_on > 0 ? 1 : 0;  // the wide classes' digit sorts
   const uint64_t per = 3 + merkle + 1 + (c->fb ? 1 + sorts : 2) + 1 + 1 + 1;
   return per * (uint64_t)nb + (c->fb ? 2 : 0);
 }
 
-// blob slot b's chunk work items: (coset, chunk, line) over the 11-bit tables,
-// for the lines without wide windows (n_l0 .. n_l0 + n_lines - 1)
-FbAccArgs blob_fb_args(const zg_ctx* c, const Lane& ln, int b = 0) {
-  const size_t R = c->R;
+// blob slot b's work items of chunk set k: (coset, unit, line) over the 11-bit tables
+FbAccArgs blob_fb_args(const zg_ctx* c, const Lane& ln, const ChunkSets& cs, int k, int b = 0) {
+  uint32_t first = 0;
+  for (int j = 0; j < k; ++j) first += chunk_set_items(c, cs.s[j]);
   FbAccArgs fa;
   fa.tab = c->tab;
-  fa.offs = ln.fb_offs + (size_t)b * 3 * R * (FB_BUCKETS + 1);
-  fa.ents = ln.fb_ents + (size_t)b * 3 * R * FB_WINDOWS * c->C;
-  fa.out = ln.fb_out + (size_t)b * blob_items(c) * FB_OUT;
-  fa.lr = c->lr;
-  fa.lc = c->lc;
-  fa.lines = c->n_lines;
-  fa.l0 = c->n_l0;
+  fa.offs = ln.fb_offs + (size_t)b * chunk_offs(c) + (size_t)chunk_units(c, cs, k) * (FB_BUCKETS + 1);
+  fa.ents = ln.fb_ents + (size_t)b * chunk_ents(c) + (size_t)k * 3 * c->N * FB_WINDOWS;
+  fa.out = ln.fb_out + ((size_t)b * blob_items(c) + first) * FB_OUT;
+  fa.lr = c->lr + c->lc - cs.s[k].ulog;
+  fa.lc = cs.s[k].ulog;
+  fa.lines = cs.s[k].nl;
+  fa.l0 = cs.s[k].l0;
   fa.Ltot = c->L;
   fa.W = FB_WINDOWS;
   fa.tabN = c->N;
   return fa;
 }
 
+// the digit sorts of blob slot b's chunk sets, one launch
+void launch_fb_sort(const zg_ctx* c, const Lane& ln, int b, const uint8_t* enc, cudaStream_t s) {
+  const ChunkSets cs = chunk_sets(c);
+  FbSortPlan p;
+  int most = 0;
+  for (int k = 0; k < cs.n; ++k) {
+    const FbAccArgs fa = blob_fb_args(c, ln, cs, k, b);
+    p.ulog[k] = fa.lc;
+    p.offs[k] = const_cast<uint32_t*>(fa.offs);
+    p.ents[k] = const_cast<uint16_t*>(fa.ents);
+    p.start[++p.n] = p.start[k] + (1u << fa.lr);
+    most = std::max(most, fa.lc);
+  }
+  k_fb_sort<<<dim3(p.start[p.n], 3), 256, fb_sort_smem_bytes(most), s>>>(enc, p, c->lr, c->lc, 1, c->N);
+}
+
+// the sort of one vector in 2^lr chunks of 2^lc points, in order
+void launch_fb_sort_single(const uint8_t* scalars, uint32_t* offs, uint16_t* ents, int lr, int lc, cudaStream_t s) {
+  FbSortPlan p;
+  p.n = 1;
+  p.start[1] = 1u << lr;
+  p.ulog[0] = lc;
+  p.offs[0] = offs;
+  p.ents[0] = ents;
+  k_fb_sort<<<dim3(1u << lr, 1), 256, fb_sort_smem_bytes(lc), s>>>(scalars, p, lr, lc, 0, 0);
+}
+
 // first item of wide class k in a blob's item order (chunk items, then the
 // classes); the sums of item u sit at fb_out + FB_OUT u
 uint32_t blob_wd_first_item(const zg_ctx* c, size_t k) {
-  uint32_t u = (uint32_t)(3 * c->R * c->n_lines);
+  uint32_t u = blob_chunk_items(c);
   for (size_t j = 0; j < k; ++j) u += (uint32_t)(3 * (c->R >> c->wd[j].mlog) * c->wd[j].nl);
   return u;
 }
@@ -928,17 +1005,21 @@ FbAccArgs blob_wd_args(const zg_ctx* c, const Lane& ln, size_t k, int b = 0) {
 // part block b
 FbCombinePlan blob_fb_plan(const zg_ctx* c, int nb = 1) {
   FbCombinePlan p;
-  const int per = 1 + c->wd_on;
+  const ChunkSets cs = chunk_sets(c);
+  const int per = cs.n + c->wd_on;
   const uint64_t part_blk = 3 * (uint64_t)c->L * c->R;
   p.n = per * nb;
   for (int b = 0; b < nb; ++b) {
     const uint32_t base = (uint32_t)b * blob_items(c);
-    p.start[per * b] = base;
-    p.m[per * b] = FbCombineMap{c->lr, c->n_lines, c->n_l0, c->L, 0, 0, 0, part_blk * b};
+    for (uint32_t k = 0, u = base; k < (uint32_t)cs.n; u += chunk_set_items(c, cs.s[k++])) {
+      const int m = cs.s[k].ulog - c->lc;  // chunks per item, log2
+      p.start[per * b + k] = u;
+      p.m[per * b + k] = FbCombineMap{c->lr - m, cs.s[k].nl, cs.s[k].l0, c->L, 0, 0, m, part_blk * b};
+    }
     for (size_t k = 0; k < (size_t)c->wd_on; ++k) {
       const zg_ctx::WdClass& w = c->wd[k];
-      p.start[per * b + 1 + k] = base + blob_wd_first_item(c, k);
-      p.m[per * b + 1 + k] =
+      p.start[per * b + cs.n + k] = base + blob_wd_first_item(c, k);
+      p.m[per * b + cs.n + k] =
           FbCombineMap{c->lr - w.mlog, w.nl, w.l0, c->L, w.hi_last, w.ulog - 10, w.mlog, part_blk * b};
     }
   }
@@ -1031,10 +1112,12 @@ FbAccPlan single_acc_plan(const FbAccArgs& fa, uint32_t units) {
 // place in the combine's item order (blob_fb_plan).
 FbAccPlan blob_acc_plan(const zg_ctx* c, const Lane& ln, int nb = 1) {
   struct Kind {
-    int k;  // wide class, or -1 for the chunk items
-    uint32_t ents;  // entries per item (windows x 1024 points)
+    int k;  // wide class, or -1 - chunk set
+    uint32_t ents;  // entries per item (windows x points per bucket block)
   };
-  std::vector<Kind> kinds{{-1, (uint32_t)FB_WINDOWS * 1024u}};
+  const ChunkSets cs = chunk_sets(c);
+  std::vector<Kind> kinds;
+  for (int k = 0; k < cs.n; ++k) kinds.push_back({-1 - k, (uint32_t)FB_WINDOWS << cs.s[k].ulog});
   for (int k = 0; k < c->wd_on; ++k)
     kinds.push_back({k, ((uint32_t)wd_windows(c->wd[k].ulog) * 1024u) << c->wd[k].mlog});
   std::stable_sort(kinds.begin(), kinds.end(), [](const Kind& x, const Kind& y) { return x.ents > y.ents; });
@@ -1044,8 +1127,8 @@ FbAccPlan blob_acc_plan(const zg_ctx* c, const Lane& ln, int nb = 1) {
     for (int b = 0; b < nb; ++b) {
       p.start[p.n] = at;
       if (kd.k < 0) {
-        p.a[p.n] = blob_fb_args(c, ln, b);
-        at += (uint32_t)(3 * c->R * c->n_lines);
+        p.a[p.n] = blob_fb_args(c, ln, cs, -1 - kd.k, b);
+        at += chunk_set_items(c, cs.s[-1 - kd.k]);
       } else {
         const zg_ctx::WdClass& w = c->wd[kd.k];
         p.a[p.n] = blob_wd_args(c, ln, (size_t)kd.k, b);
@@ -1085,19 +1168,24 @@ int launch_sum_points(const XYZZ* in, uint32_t n, uint64_t stride, uint32_t sets
 constexpr int FS_MAX_LOG = 15;
 uint32_t fs_splits(int logn) { return logn > FS_MAX_LOG ? 0 : 1u << std::max(0, logn - 12); }
 
-// k_wd_sort / k_wd_tables for a class's unit size
-void launch_wd_sort(int ulog, const uint8_t* enc, uint32_t* offs, uint32_t* ents, int lr, int lc, size_t N,
-                    cudaStream_t s) {
-  const dim3 grid((unsigned)(N >> ulog), 3);
-  const size_t sm = wd_sort_smem_bytes(ulog);
-  switch (ulog) {
-    case 15: k_wd_sort<15><<<grid, WD_SORT_THREADS, sm, s>>>(enc, offs, ents, lr, lc, 1, N); break;
-    case 14: k_wd_sort<14><<<grid, WD_SORT_THREADS, sm, s>>>(enc, offs, ents, lr, lc, 1, N); break;
-    case 13: k_wd_sort<13><<<grid, WD_SORT_THREADS, sm, s>>>(enc, offs, ents, lr, lc, 1, N); break;
-    case 12: k_wd_sort<12><<<grid, WD_SORT_THREADS, sm, s>>>(enc, offs, ents, lr, lc, 1, N); break;
-    default: k_wd_sort<11><<<grid, WD_SORT_THREADS, sm, s>>>(enc, offs, ents, lr, lc, 1, N); break;
+// the digit sorts of the first `on` wide classes for blob slot b, one launch
+// with the largest units first (nothing without wide classes)
+void launch_wd_sort(const zg_ctx* c, const Lane& ln, int on, int b, const uint8_t* enc, cudaStream_t s) {
+  WdSortPlan p;
+  size_t smem = 0;
+  for (int k = 0; k < on; ++k) {
+    if (c->wd[k].sort_of != k) continue;
+    p.ulog[p.n] = c->wd[k].ulog;
+    p.offs[p.n] = lane_wd_offs(c, ln, (size_t)k, b);
+    p.ents[p.n] = lane_wd_ents(c, ln, (size_t)k, b);
+    p.start[p.n + 1] = p.start[p.n] + (uint32_t)(c->N >> c->wd[k].ulog);
+    ++p.n;
+    smem = std::max(smem, wd_sort_smem_bytes(c->wd[k].ulog));
   }
+  if (p.n) k_wd_sort<<<dim3(3, p.start[p.n]), WD_SORT_THREADS, smem, s>>>(enc, p, c->lr, c->lc, c->N);
 }
+
+// k_wd_tables for a class's unit size
 void launch_wd_tables(const zg_ctx* c, const zg_ctx::WdClass& k, cudaStream_t s) {
   const unsigned g = nblk((uint64_t)3 * k.nl * c->N, 128);
   switch (k.ulog) {
@@ -1157,12 +1245,8 @@ int encode_launches(zg_ctx* c, const Lane& ln, const BlobBufs* b, int nb, const 
   // AMT: MSM items of every blob, trees, serialisation
   if (c->fb) {
     for (int i = 0; i < nb; ++i) {
-      const FbAccArgs fa = blob_fb_args(c, ln, i);
-      k_fb_sort<<<dim3((unsigned)R, 3), 256, fb_sort_smem_bytes(lc), s>>>(b[i].enc, const_cast<uint32_t*>(fa.offs),
-                                                                           const_cast<uint16_t*>(fa.ents), lr, lc, 1, N);
-      for (size_t k = 0; k < (size_t)c->wd_on; ++k)
-        if (c->wd[k].sort_of == (int)k)
-          launch_wd_sort(c->wd[k].ulog, b[i].enc, lane_wd_offs(c, ln, k, i), lane_wd_ents(c, ln, k, i), lr, lc, N, s);
+      launch_fb_sort(c, ln, i, b[i].enc, s);
+      launch_wd_sort(c, ln, c->wd_on, i, b[i].enc, s);
     }
   }
   }  // PHASE_PRE
@@ -2168,8 +2252,7 @@ int verify_msms(VerifyRun& v, const bool present[3], XYZZ* out) {
     FbAccArgs& fa = acc.a[k];
     uint32_t* offs = c->lane.fb_offs + (size_t)k * R * (FB_BUCKETS + 1);
     uint16_t* ents = c->lane.fb_ents + (size_t)k * R * FB_WINDOWS * c->C;
-    k_fb_sort<<<dim3(R, 1), 256, fb_sort_smem_bytes(c->lc), v.s>>>(v.d_scal + (size_t)cs * c->N * 32, offs, ents, c->lr,
-                                                                   c->lc, 0, 0);
+    launch_fb_sort_single(v.d_scal + (size_t)cs * c->N * 32, offs, ents, c->lr, c->lc, v.s);
     fa.tab = c->line_ptr(cs, c->lr);
     fa.offs = offs;
     fa.ents = ents;
@@ -3042,13 +3125,8 @@ int zg_ctx_autotune(zg_ctx* c, zg_tuning* out) {
     // the whole blob MSM (digit sorts, bucket accumulation, combine) with the
     // first j wide classes, product kind `kind`
     auto full_msm = [&](uint32_t kind, int j) {
-      const FbAccArgs f0 = blob_fb_args(c, c->lane);
-      k_fb_sort<<<dim3((unsigned)c->R, 3), 256, fb_sort_smem_bytes(c->lc), s>>>(
-          c->enc, const_cast<uint32_t*>(f0.offs), const_cast<uint16_t*>(f0.ents), c->lr, c->lc, 1, c->N);
-      for (int k = 0; k < j; ++k)
-        if (c->wd[k].sort_of == k)
-          launch_wd_sort(c->wd[k].ulog, c->enc, lane_wd_offs(c, c->lane, k, 0), lane_wd_ents(c, c->lane, k, 0), c->lr,
-                         c->lc, c->N, s);
+      launch_fb_sort(c, c->lane, 0, c->enc, s);
+      launch_wd_sort(c, c->lane, j, 0, c->enc, s);
       launch_fb_accum(c, c->lane, kind, blob_acc_plan(c, c->lane, 1), s);
       launch_fb_combine(c->lane, blob_fb_plan(c, 1), s);
     };
@@ -3325,8 +3403,7 @@ int zg_ctx_msm(zg_ctx* c, uint32_t coset, uint32_t line, const void* d_scalars, 
   ZG_CK(cudaSetDevice(c->device));
   cudaStream_t s = (cudaStream_t)stream;
   ZG_CK(cudaStreamWaitEvent(s, c->done, 0));
-  k_fb_sort<<<dim3(nch, 1), 256, fb_sort_smem_bytes(lcs), s>>>((const uint8_t*)d_scalars, c->lane.fb_offs, c->lane.fb_ents,
-                                                                lrn, lcs, 0, 0);
+  launch_fb_sort_single((const uint8_t*)d_scalars, c->lane.fb_offs, c->lane.fb_ents, lrn, lcs, s);
   if (splits) {
     // (T, S) of every group and split go to the bucket kernel's scratch
     XYZZ* ts = reinterpret_cast<XYZZ*>(c->lane.fb_scratch.base);

@@ -579,27 +579,44 @@ __device__ __forceinline__ uint32_t fb_window_bits(const uint32_t* s, int w) {
   return v & ((1u << FB_BITS) - 1);
 }
 
-// Per chunk: counting sort of the (point, window) pairs by |digit|.
+constexpr int FB_MAX_CHUNK_SETS = 8;  // sets of 11-bit items of a blob (more than one: no wide classes)
+// The units that one k_fb_sort launch sorts: set k's blocks start[k] ..
+// start[k + 1] - 1 take the units of 2^ulog[k] points of one vector per
+// blockIdx.y, units[k] per vector
+struct FbSortPlan {
+  int n = 0;
+  uint32_t start[FB_MAX_CHUNK_SETS + 1] = {};
+  int ulog[FB_MAX_CHUNK_SETS] = {};
+  uint32_t* offs[FB_MAX_CHUNK_SETS] = {};
+  uint16_t* ents[FB_MAX_CHUNK_SETS] = {};
+};
+
+// Per unit (a chunk, or consecutive chunks of fewer than 1024 points that
+// share an item's buckets): counting sort of the (point, window) pairs by |digit|.
 //   offs[g][k-1] .. offs[g][k]  = entries of bucket k (k = 1..1024)
 //   ents[g][e] = t | w << 10 | sign << 15
-// g = coset * nchunks + chunk. Chunk b reads encoded row bitrev(b), element t
-// = column bitrev(t) when bitrev_rows is set (HalfBlob::generate's index_reverse).
-__global__ void __launch_bounds__(256) k_fb_sort(const uint8_t* __restrict__ scalars, uint32_t* __restrict__ offs,
-                                                 uint16_t* __restrict__ ents, int lr, int lc, int bitrev_rows,
-                                                 uint64_t scalar_coset_stride) {
+// g = coset * units + unit, t < 2^ulog the point in the unit. Chunk b reads
+// encoded row bitrev(b), its point t = column bitrev(t) when bitrev_rows is set
+// (HalfBlob::generate's index_reverse).
+__global__ void __launch_bounds__(256) k_fb_sort(const uint8_t* __restrict__ scalars, const FbSortPlan plan, int lr,
+                                                 int lc, int bitrev_rows, uint64_t scalar_coset_stride) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int C = 1 << lc;
-  const uint32_t b = blockIdx.x, coset = blockIdx.y;
-  const uint32_t g = coset * (1u << lr) + b;
+  int set = 0;
+  while (set + 1 < plan.n && blockIdx.x >= plan.start[set + 1]) ++set;
+  const int C = 1 << plan.ulog[set];
+  const uint32_t unit = blockIdx.x - plan.start[set], units = plan.start[set + 1] - plan.start[set];
+  const uint32_t coset = blockIdx.y, g = coset * units + unit;
+  uint32_t* const offs = plan.offs[set];
+  uint16_t* const ents = plan.ents[set];
   uint32_t* scal = reinterpret_cast<uint32_t*>(smem);            // [C][8]
   uint32_t* cnt = scal + (size_t)C * 8;                           // [FB_BUCKETS + 1]
   uint32_t* part = cnt + FB_BUCKETS + 1;                          // [256]
   uint16_t* lst = reinterpret_cast<uint16_t*>(part + 256);        // [W * C]
-  const uint32_t row = bitrev_rows ? brev_bits(b, lr) : b;
-  const uint8_t* src = scalars + (scalar_coset_stride * coset + (uint64_t)row * C) * 32;
+  const uint8_t* src = scalars + scalar_coset_stride * coset * 32;
   for (int t = threadIdx.x; t < C; t += blockDim.x) {
-    uint32_t col = bitrev_rows ? brev_bits(t, lc) : t;
-    const uint4* q = reinterpret_cast<const uint4*>(src + (size_t)col * 32);
+    const uint32_t p = (unit << plan.ulog[set]) + t, b = p >> lc, e = p & ((1u << lc) - 1);
+    const uint32_t row = bitrev_rows ? brev_bits(b, lr) : b, col = bitrev_rows ? brev_bits(e, lc) : e;
+    const uint4* q = reinterpret_cast<const uint4*>(src + (((uint64_t)row << lc) + col) * 32);
     uint4 x = q[0], y = q[1];
     uint32_t* d = scal + (size_t)t * 8;
     d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w; d[4] = y.x; d[5] = y.y; d[6] = y.z; d[7] = y.w;
@@ -665,14 +682,6 @@ __global__ void __launch_bounds__(256) k_fb_sort(const uint8_t* __restrict__ sca
 constexpr int WD_SORT_THREADS = 1024;
 inline size_t wd_sort_smem_bytes(int ulog) { return (size_t)((1u << ulog) + 1 + 32) * sizeof(uint32_t); }
 
-// Per sort unit of U = 2^ULOG consecutive points of a coset (chunks
-// u U / 1024 .. (u + 1) U / 1024 - 1 of 1024 columns): counting sort of the
-// (point, window) pairs by |digit| of the signed c = ULOG + 1 bit digits.
-//   offs[cs][u][k] .. offs[cs][u][k + 1] = entries of bucket k (|digit| = k + 1)
-//   ents[cs][u][e] = p | w << ULOG | sign << 31, p the point within the unit
-// Point p of unit u is chunk b = (u U + p) >> lc, element t = (u U + p) &
-// (2^lc - 1), read like k_fb_sort reads it. Pass 1 counts, a block scan turns
-// the counts into fill pointers, pass 2 scatters (the scalars are read twice).
 template <int C>
 __device__ __forceinline__ uint32_t wd_window_bits(const uint32_t* s, int w) {
   const int o = C * w;
@@ -682,18 +691,25 @@ __device__ __forceinline__ uint32_t wd_window_bits(const uint32_t* s, int w) {
   return v & ((1u << C) - 1);
 }
 
+// Per sort unit of U = 2^ULOG consecutive points of a coset (chunks
+// u U / 1024 .. (u + 1) U / 1024 - 1 of 1024 columns): counting sort of the
+// (point, window) pairs by |digit| of the signed c = ULOG + 1 bit digits.
+//   offs[cs][u][k] .. offs[cs][u][k + 1] = entries of bucket k (|digit| = k + 1)
+//   ents[cs][u][e] = p | w << ULOG | sign << 31, p the point within the unit
+// Point p of unit u is chunk b = (u U + p) >> lc, element t = (u U + p) &
+// (2^lc - 1), read like k_fb_sort reads it. Pass 1 counts, a block scan turns
+// the counts into fill pointers, pass 2 scatters (the scalars are read twice).
+// (the rows and columns in bit-reversed order).
 template <int ULOG>
-__global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __restrict__ scalars,
-                                                             uint32_t* __restrict__ offs, uint32_t* __restrict__ ents,
-                                                             int lr, int lc, int bitrev_rows,
-                                                             uint64_t scalar_coset_stride) {
+__device__ __forceinline__ void wd_sort_unit(const uint8_t* __restrict__ scalars, uint32_t* __restrict__ offs,
+                                             uint32_t* __restrict__ ents, uint32_t unit, uint32_t coset,
+                                             uint32_t nunits, int lr, int lc, uint64_t scalar_coset_stride) {
   constexpr int C = ULOG + 1, W = wd_windows(ULOG);
   constexpr uint32_t U = 1u << ULOG, NB = U;           // buckets = 2^(c - 1) = U
   constexpr int PER = (int)NB / WD_SORT_THREADS;       // counters per thread in the scan
   static_assert(PER >= 1, "at least 1024 buckets");
   extern __shared__ __align__(16) uint32_t wcnt[];     // [NB + 1], then [32] warp sums
   uint32_t* wsum = wcnt + NB + 1;
-  const uint32_t unit = blockIdx.x, coset = blockIdx.y, nunits = gridDim.x;
   const uint32_t Cn = 1u << lc;
   const uint8_t* src = scalars + scalar_coset_stride * coset * 32;
   uint32_t* o = offs + ((size_t)coset * nunits + unit) * (NB + 1);
@@ -704,8 +720,7 @@ __global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __re
     for (uint32_t p = threadIdx.x; p < U; p += blockDim.x) {
       const uint32_t gp = (unit << ULOG) + p;
       const uint32_t b = gp >> lc, t = gp & (Cn - 1);
-      const uint32_t row = bitrev_rows ? brev_bits(b, lr) : b;
-      const uint32_t col = bitrev_rows ? brev_bits(t, lc) : t;
+      const uint32_t row = brev_bits(b, lr), col = brev_bits(t, lc);
       const uint4* q = reinterpret_cast<const uint4*>(src + ((uint64_t)row * Cn + col) * 32);
       const uint4 x = q[0], y = q[1];
       const uint32_t s[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
@@ -759,6 +774,32 @@ __global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __re
   }
 }
 
+// The sorts of a blob's wide classes in one launch: class k's units are blocks
+// start[k] .. start[k + 1] - 1 of each coset, largest units first. A block of
+// the largest unit holds an SM for 465 us whatever the others do (1024 threads
+// and 128 KB), and a 128 x 1024 blob has 12 of them, 24 of the next size and so
+// on: one launch after another took 990 us there, together some 500.
+struct WdSortPlan {
+  int n = 0;
+  uint32_t start[FB_MAX_CHUNK_SETS + 1] = {};
+  int ulog[FB_MAX_CHUNK_SETS] = {};
+  uint32_t* offs[FB_MAX_CHUNK_SETS] = {};
+  uint32_t* ents[FB_MAX_CHUNK_SETS] = {};
+};
+__global__ void __launch_bounds__(WD_SORT_THREADS) k_wd_sort(const uint8_t* __restrict__ scalars, const WdSortPlan plan,
+                                                             int lr, int lc, uint64_t scalar_coset_stride) {
+  int k = 0;
+  while (k + 1 < plan.n && blockIdx.y >= plan.start[k + 1]) ++k;
+  const uint32_t unit = blockIdx.y - plan.start[k], nunits = plan.start[k + 1] - plan.start[k], coset = blockIdx.x;
+  switch (plan.ulog[k]) {
+    case 15: wd_sort_unit<15>(scalars, plan.offs[k], plan.ents[k], unit, coset, nunits, lr, lc, scalar_coset_stride); break;
+    case 14: wd_sort_unit<14>(scalars, plan.offs[k], plan.ents[k], unit, coset, nunits, lr, lc, scalar_coset_stride); break;
+    case 13: wd_sort_unit<13>(scalars, plan.offs[k], plan.ents[k], unit, coset, nunits, lr, lc, scalar_coset_stride); break;
+    case 12: wd_sort_unit<12>(scalars, plan.offs[k], plan.ents[k], unit, coset, nunits, lr, lc, scalar_coset_stride); break;
+    default: wd_sort_unit<11>(scalars, plan.offs[k], plan.ents[k], unit, coset, nunits, lr, lc, scalar_coset_stride); break;
+  }
+}
+
 }  // namespace zg
 #include "zg_bucket.cuh"
 #include "zg_quad.cuh"
@@ -775,8 +816,8 @@ __device__ __forceinline__ void store_g1(const XYZZ& p, uint8_t* out) {
 }
 
 // Where a combine launch's items go. The launch covers up to FB_MAX_SETS item
-// sets (the chunk items, then one set per wide unit size); set k holds items
-// start[k] .. start[k + 1] - 1, whose (T, S) partials sit at the same
+// sets (the chunk sets, then one set per wide unit size); set k holds items
+// start[k] .. start[k + 1] - 1, whose row and column sums sit at the same
 // positions. Local item v = u - start[k] of line l = v % lines (g = v / lines,
 // coset g >> lr, b = g & (2^lr - 1)) is written to part[(coset * L + line) *
 // 2^lr + b], line = L - 1 for the set's last line when hi_last, else l0 + l.
@@ -784,8 +825,9 @@ __device__ __forceinline__ void store_g1(const XYZZ& p, uint8_t* out) {
 // sum_k B_k: their buckets hold digits 1024 blk + k + 1 (bpu_log = 0 for
 // chunk items). part_off places a fused launch's blob in its own part block.
 // lr: log2 of the set's items per (coset, line); a wide set's items are
-// blocks of 2^bpu_log per unit, and a merged unit (mlog = 1) spans 2^(bpu_log
-// + mlog) part slots (one per 1024 points): its items fill the first 2^bpu_log
+// blocks of 2^bpu_log per unit, and a merged unit (mlog > 0: two sort units, or
+// 2^mlog chunks of fewer than 64 points) spans 2^(bpu_log + mlog) part slots
+// (one per chunk): its items fill the first 2^bpu_log
 // and the identity the rest, so the AMT trees sum every line's R slots alike.
 struct FbCombineMap {
   int lr, lines, l0, L, hi_last, bpu_log, mlog;

@@ -740,3 +740,15 @@ def test_merkle_levels_match_oracle(gpu_pkg, oracle, log_per_root):
     # 3 roots of 2^k leaves of 8 items: a blob of 2^(k - 4) rows of 128 columns has the same tree
     lr, lc = (log_per_root, 3) if log_per_root < 8 else (log_per_root - 7, 10)
     assert host(out) == oracle.merkle_roots(lr, lc, items)
+
+
+@pytest.mark.parametrize("log_row,log_col", [(1, 3), (2, 3), (7, 3), (5, 4), (1, 5), (6, 5)])
+def test_encode_merged_units_match_oracle(gpu_pkg, oracle, log_row, log_col):
+    """Contexts of fewer than 64 columns, whose MSM items take several chunks:
+    nodes smaller than, equal to and larger than the largest unit."""
+    params = gpu_pkg.ZgEncoderParams.from_seed(log_row, log_col, 3)
+    op = oracle.params(log_row, log_col, 3)
+    rng = np.random.default_rng(log_row * 16 + log_col)
+    for n in (1, params.dims.max_raw_data_size):
+        _check_against_oracle(gpu_pkg, oracle, params, op, rng.integers(0, 256, n, dtype=np.uint8).tobytes())
+    params.close()
