@@ -427,20 +427,19 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     __syncthreads();  // every thread has read the previous group number
     if (tid == 0) item = atomicAdd(next, 1u);
     __syncthreads();
-    // group number -> set and its items u0 .. u0 + ng - 1
-    uint32_t u0 = item;
+    // group number -> set and its items u0, u0 + groups, ..: spread over the set,
+    // as neighbours may all be empty (a scalar vector's zero end) or all full
+    uint32_t u0 = item, groups = 0;
     int set = 0;
     for (; set < plan.n; ++set) {
       const uint32_t group = (uint32_t)plan.a[set].group;
-      const uint32_t groups = (plan.start[set + 1] - plan.start[set] + group - 1) / group;
+      groups = (plan.start[set + 1] - plan.start[set] + group - 1) / group;
       if (u0 < groups) break;
       u0 -= groups;
     }
     if (set >= plan.n) break;
     const FbAccArgs& a = plan.a[set];
-    const uint32_t group = (uint32_t)a.group;
-    u0 *= group;
-    const uint32_t ng = min(group, plan.start[set + 1] - plan.start[set] - u0);
+    const uint32_t ng = (plan.start[set + 1] - plan.start[set] - u0 + groups - 1) / groups;
     const bool wide = a.ents32 != nullptr;
     // item i of the group: its bucket offsets, entries and first table point
     struct Item {
@@ -449,7 +448,7 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
       uint32_t tab;
     };
     auto item_of = [&](uint32_t i) {
-      const uint32_t u = u0 + i, nch = 1u << a.lr;
+      const uint32_t u = u0 + i * groups, nch = 1u << a.lr;
       const uint32_t l = u % a.lines, g = u / a.lines;
       const uint32_t coset = g / nch, b = g % nch;
       Item it;
@@ -640,7 +639,7 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     // R_a in slot 16 a, C_b in slot 512 + b of the item's slots
     for (uint32_t k = tid; k < ng * FB_OUT; k += T) {
       const uint32_t i = k / FB_OUT, o = k % FB_OUT;
-      st_aff(a.out + (size_t)(u0 + i) * FB_OUT + o,
+      st_aff(a.out + (size_t)(u0 + i * groups) * FB_OUT + o,
              ld_aff(slots + i * FB_BUCKETS + (o < FB_GRID ? o * (FB_GRID / 2) : FB_BUCKETS / 2 + o - FB_GRID)));
     }
   }
