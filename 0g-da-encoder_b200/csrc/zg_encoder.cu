@@ -3355,7 +3355,7 @@ int zg_recover(zg_ctx* c, const uint64_t* row_ids, const uint8_t* const* rows, c
                                                        c->rec_ginv, c->tw.wni_lo, c->tw.wni_hi, c->rec_err);
   k_rec_zinv<<<nblk(M, 32), 32 * REC_Z_WARPS, 0, s>>>(c->rec_erased, (uint32_t)erased.size(), c->rec_wpow, host_fr_from_u32(5),
                                           c->rec_zw, c->rec_zinv, (uint32_t)M);
-  k_rec_cols<<<(unsigned)C, REC_COL_THREADS, (M + R) * sizeof(Fr), s>>>(c->rec_V, c->rec_W, lr, lc, tm->twf_c, tm->twi_c,
+  k_rec_cols<<<(unsigned)C, rec_col_threads(M), (M + R) * sizeof(Fr), s>>>(c->rec_V, c->rec_W, lr, lc, tm->twf_c, tm->twi_c,
                                                              c->rec_kpow, c->rec_kinv, c->rec_zw, c->rec_zinv, c->tw.twf_r,
                                                              c->tw.wn_lo, c->tw.wn_hi, c->rec_err);
   k_rec_out<<<(unsigned)R, 256, C * sizeof(Fr), s>>>(c->rec_W, c->rec_raw, lc, c->tw.twf_c, c->rec_err);

@@ -92,9 +92,15 @@ __global__ void __launch_bounds__(32 * REC_Z_WARPS) k_rec_zinv(const uint16_t* _
   }
 }
 
-// Threads per column: the 5 R x 32 bytes of shared memory leave one CTA per SM
-// at R = 1024, so its own warps have to keep the SM busy (2.23 ms at 256, 2.10 at 512).
+// Threads per column: one per radix-4 group of the 4R-point transforms (M / 4),
+// so that no warp waits at barriers without work and small R leaves several
+// CTAs per SM (512 threads throughout cost 0.4 ms of a 128 x 1024 recovery's
+// 2.7). At R = 1024 the 5 R x 32 bytes of shared memory leave one CTA per SM,
+// whose own warps have to keep it busy (2.23 ms at 256 threads, 2.10 at 512).
 constexpr int REC_COL_THREADS = 512;
+inline unsigned rec_col_threads(size_t M) {
+  return (unsigned)(M / 4 < 64 ? 64 : M / 4 > REC_COL_THREADS ? REC_COL_THREADS : M / 4);
+}
 // Per column s: decode P_s from its 4R samples (zeros at erased points), then
 // W_out[r][s] = w^{r s} P_s(W^{4r}). err bit 1: a coefficient >= R is nonzero
 // (the rows are not one codeword).
