@@ -108,18 +108,25 @@ def executed_mixed_adds(lr, lc, wide_classes=6):
     return total
 
 
+def executed_grid_adds(lr, lc, wide_classes=6):
+    """Affine additions of the bucket grids per blob: per MSM work item (1024
+    buckets each: 3 x rows per line, half as many on the lines of 2^16-point
+    units) 31 additions in each of its 32 rows and 32 columns."""
+    return _executed_items(lr, lc, wide_classes) * 64 * 31
+
+
 def executed_full_adds(lr, lc, wide_classes=6):
-    """XYZZ + XYZZ additions of the bucket reductions per blob: per MSM work
-    item (1024 buckets each: 3 x rows per line, half as many on the lines of
-    2^16-point units) the running sums of its 128 threads (two per bucket;
-    the merges of a bucket's extra task partials are not counted) and the
-    combine of the 128 (T, S) partials (2 x 127 additions plus 3
-    doublings)."""
+    """XYZZ additions of the combine per blob: running sums over the 64 row and
+    column sums of each item, and 5 doublings."""
+    return _executed_items(lr, lc, wide_classes) * (126 + 5)
+
+
+def _executed_items(lr, lc, wide_classes):
     items = 0
     for lg, u in _line_unit_logs(lr, lc):
         merged = _wide(lc, lg, u, wide_classes) and u == 16
         items += 3 * ((1 << lr) >> (1 if merged else 0))
-    return items * (2 * 1024 + 2 * 127 + 3)
+    return items
 
 
 def ntt_muls(logn):
@@ -132,18 +139,17 @@ def ntt_muls(logn):
 
 def zg_ntt_products(batch, logn, inverse, coset):
     """Fr products of one zg_ntt call: up to 2^11 points one transform per
-    vector (coset shift 1 product per element from a full table, 1/n 1
-    product); above, the four-step split (lc = ceil(logn / 2)): column
-    transforms, 2 products per element for the twiddles between the passes,
-    row transforms (coset shift 2 products per element from split tables)."""
+    vector (1/n 1 product per element); above, the four-step split (lc =
+    ceil(logn / 2)): column transforms, 1 product per element for the twiddles
+    between the passes (1/n inside them), row transforms. A coset shift is 1
+    product per element."""
     n = 1 << logn
     if logn <= 11:
         per = ntt_muls(logn) + (n if coset else 0) + (n if inverse else 0)
     else:
         lc = (logn + 1) // 2
         lr = logn - lc
-        per = (1 << lc) * ntt_muls(lr) + 2 * n + (1 << lr) * ntt_muls(lc) \
-            + (2 * n if coset else 0) + (n if inverse else 0)
+        per = (1 << lc) * ntt_muls(lr) + n + (1 << lr) * ntt_muls(lc) + (n if coset else 0)
     return batch * per
 
 
@@ -840,7 +846,8 @@ def main():
     wide_on = tuning.get("msm_wide_classes", 6)
     ex_mixed = executed_mixed_adds(LOG_ROW, LOG_COL, wide_on)
     ex_full = executed_full_adds(LOG_ROW, LOG_COL, wide_on)
-    ex_prod = ex_mixed * 10 + ex_full * 14
+    ex_grid = executed_grid_adds(LOG_ROW, LOG_COL, wide_on)
+    ex_prod = (ex_mixed + ex_grid) * 6 + ex_full * 14
     ex_imad = ex_prod * 264
     prod_by_kind = {k: pkg.probe_products(local, k) for k in pkg.MSM_PRODUCTS}
     prod_peak = prod_by_kind[tuning.get("msm_product", "hybrid")]
@@ -849,20 +856,20 @@ def main():
         "frac": achieved / imad, "traffic": profile_traffic(),
         "note": "work = 1509949440 mixed adds/blob x 10 Fq mul x 264 IMAD (reference decomposition; "
                 f"this build executes {ex_mixed} table-point additions plus "
-                "the bucket reductions, half of the products on the FP64 pipe, so frac may exceed 1); "
+                "the bucket grids, affine with shared inversions, so frac may exceed 1); "
                 "peak = live mad.lo.u32 probe on this GPU (of measured); traffic = dram bytes per launch "
                 "from the committed ncu summary",
-        "executed_mixed_adds": ex_mixed, "executed_full_adds": ex_full,
+        "executed_mixed_adds": ex_mixed, "executed_grid_adds": ex_grid, "executed_full_adds": ex_full,
         "executed_frac": ex_imad / t_msm / 1e9 / imad,
         "executed_products_per_s": ex_prod / t_msm,
         "product_peak_per_s": prod_peak * 1e9,
         "product_frac": ex_prod / t_msm / 1e9 / prod_peak,
         "product_probe_by_kind": {k: v * 1e9 for k, v in prod_by_kind.items()},
-        "product_note": "executed Fq products (mixed additions x 10 + XYZZ additions x 14) per second of the MSM "
+        "product_note": "executed Fq products (affine additions x 6 + XYZZ additions x 14) per second of the MSM "
                         "phase / the live product-throughput probe of the same product kind at the bucket "
                         "kernel's launch shape (zg_probe_products): how close the bucket loop runs to the rate "
                         "its field products can be issued",
-        "executed_note": "the additions this build runs (mixed x 10 Fq products + XYZZ x 14) x 264 IMAD per "
+        "executed_note": "the additions this build runs (affine x 6 Fq products + XYZZ x 14) x 264 IMAD per "
                          "product / MSM phase time / the live IMAD probe: a utilisation of the integer pipe as if "
                          "every product ran there (the FP64-pipe share of the hybrid kinds counts as IMAD work)",
     }

@@ -111,9 +111,8 @@ int zg_ctx_param_points(zg_ctx* ctx, int coset, int line, size_t first, size_t c
  *                    column sums (wide multiply-adds, no carry flags),
  *                    ZG_MSM_PRODUCT_W28_HYBRID one of those and one on the FP64
  *                    pipe;
- *   msm_task         bucket layout: entries per bucket-accumulation task, 32,
- *                    48, 64 (default) or 96 (buckets are cut into tasks of at
- *                    most this many points, scheduled by size);
+ *   msm_task         bucket accumulation: 32, 48, 64 (default) or 96; a thread
+ *                    makes up to 3/2 of it additions per shared inversion;
  *   msm_wide_classes MSM window width per AMT line: how many of the context's
  *                    wide-window classes are in use, largest unit first (class
  *                    u gives the lines whose nodes hold >= 2^u points units of
