@@ -75,6 +75,15 @@ static_assert(FB_GRID * FB_GRID == FB_BUCKETS, "buckets fill the grid");
 // levels of their trees run together, so the short levels share their
 // inversions.
 constexpr int FB_GROUP = 4;
+// A level's list is written by the threads that own the buckets, but runs of
+// FB_RUN_PAIRS additions or more of one bucket by the whole CTA, up to
+// FB_RUNS_MAX a level (the owner lists what is beyond): equal digits put
+// thousands of entries into one bucket. A 128 x 1024 blob of one byte repeated
+// (all digits of all windows equal) takes 46 ms, 97 listed by the owners, of
+// one element repeated 15.5 and 19.4 ms; a 1024 x 1024 one 144 and 206, 111 and
+// 126 ms. Lines of 32 to 160 pairs time alike.
+constexpr uint32_t FB_RUN_PAIRS = 64;
+constexpr uint32_t FB_RUNS_MAX = 192;
 // Per-CTA scratch, for segments of at most `cap` entries.
 struct FbScratch {
   uint8_t* base = nullptr;
@@ -254,6 +263,162 @@ __device__ __forceinline__ Fq fq_of(const uint4& a, const uint4& b) {
   return r;
 }
 
+// A work item's sort output: its bucket offsets and first entry (in elements
+// of the set's entries) for each of its sort units, and the table point of
+// index 0 and window 0
+struct BktItem {
+  const uint32_t *offs, *offs2;
+  uint32_t ents, ents2, tab;
+};
+// The lists of a set's items as k_fb_sort (16-bit entries, U) or k_wd_sort (32)
+// wrote them: lg bits of point index, then 5 of the window, the sign on top
+template <class U>
+struct BktLists {
+  const U* ents;
+  uint32_t lg, N;
+  // table point and sign bit of entry e; tab: point of index 0 and window 0
+  __device__ __forceinline__ uint32_t point(uint32_t tab, uint32_t e) const {
+    const uint32_t v = ents[e], sign = sizeof(U) == 4 ? v & 0x80000000u : (v & 0x8000u) << 16;
+    return (tab + ((v >> lg) & 31) * N + (v & ((1u << lg) - 1))) | sign;
+  }
+};
+// What a CTA lists a level with (shared memory). A run: entry or slot of its
+// first addition, its tab, number of additions, place in the list | first
+// target slot << 16
+struct BktShared {
+  uint16_t sstart[FB_GROUP * FB_BUCKETS + 1];  // first slot of each bucket
+  uint32_t wsum[FB_ACC_THREADS / 32];
+  uint4 run[FB_RUNS_MAX];
+  uint32_t runs;
+  __device__ __forceinline__ bool defer(uint32_t from, uint32_t tab, uint32_t pairs, uint32_t at, uint32_t slot) {
+    const uint32_t i = atomicAdd(&runs, 1u);
+    if (i < FB_RUNS_MAX) run[i] = make_uint4(from, tab, pairs, at | slot << 16);
+    return i < FB_RUNS_MAX;
+  }
+};
+// The listings are functions of their own: inlined, they cost the passes
+// registers (a 1024 x 1024 blob of random bytes 107.2 -> 109.2 ms; so 107.7).
+// Two pairs are listed at a time, as the stores keep the loads of the next
+// pair behind them (32 x 1024 4.95 -> 4.75 ms).
+// Level 1 of entries lo .. hi - 1 of the turn, buckets k0 .. k0 + per - 1 of
+// item `it`, whose first entry is the turn's entry `first` (`mine` false: no
+// such item): lists the pairs, writes what is alone in its bucket, and sets
+// sstart. Returns the number of additions.
+template <class U>
+static __device__ __noinline__ uint32_t bkt_list_first(BktShared& sh, const BktLists<U> l, const BktItem it, bool mine,
+                                                       uint32_t first, uint32_t lo, uint32_t hi, uint32_t k0,
+                                                       uint32_t per, const G1Aff* tab, G1Aff* slots, const G1Aff* fin,
+                                                       uint2* list, uint32_t* dst) {
+  const uint32_t f0 = it.offs[0], f1 = it.offs2 ? it.offs2[0] : 0u;
+  // the range of the segment in bucket k, as entry ranges of its two sort units
+  struct Part {
+    uint32_t e[2], n[2], carry;
+  };
+  auto part = [&](uint32_t k) {
+    Part p = {};
+    if (!mine) return p;
+    const uint32_t b = k % FB_BUCKETS;
+    const uint32_t o0 = it.offs[b], c0 = it.offs[b + 1] - o0;
+    const uint32_t o1 = it.offs2 ? it.offs2[b] : 0u, c1 = it.offs2 ? it.offs2[b + 1] - o1 : 0u;
+    const uint32_t at = first + (o0 - f0) + (o1 - f1);
+    const uint32_t qa = min(max(lo, at) - at, c0 + c1), qb = hi > at ? max(qa, min(hi - at, c0 + c1)) : qa;
+    const uint32_t a0 = min(qa, c0), b0 = min(qb, c0);
+    p.e[0] = it.ents + o0 + a0;
+    p.n[0] = b0 - a0;
+    p.e[1] = it.ents2 + o1 + (qa - a0);
+    p.n[1] = (qb - b0) - (qa - a0);
+    p.carry = at < lo && qb > qa;  // the bucket began in an earlier segment
+    return p;
+  };
+  if (threadIdx.x == 0) sh.runs = 0;  // its last readers are behind a barrier, the next ones behind block_scan's
+  uint32_t cnt = 0;  // pairs | slots << 16
+  for (uint32_t k = k0; k < k0 + per; ++k) {
+    const Part p = part(k);
+    cnt += ((p.n[0] >> 1) + (p.n[1] >> 1)) + ((((p.n[0] + 1) >> 1) + ((p.n[1] + 1) >> 1) + p.carry) << 16);
+  }
+  uint32_t total;
+  const uint32_t at = block_scan(cnt, sh.wsum, &total);
+  uint32_t p = at & 0xffffu, sl = at >> 16;
+  for (uint32_t k = k0; k < k0 + per; ++k) {
+    const Part r = part(k);
+    sh.sstart[k] = (uint16_t)sl;
+    if (r.carry) st_aff(slots + sl++, ld_aff(fin + k));
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const uint32_t pairs = r.n[s] >> 1, ptab = it.tab + (s ? 1u << l.lg : 0u);
+      uint32_t e = r.e[s];
+      if (pairs >= FB_RUN_PAIRS && sh.defer(e, ptab, pairs, p, sl)) {
+        p += pairs;
+        sl += pairs;
+        e += 2 * pairs;
+      } else {
+        uint32_t i = 0;
+        for (; i + 1 < pairs; i += 2, e += 4, p += 2, sl += 2) {
+          const uint2 x = make_uint2(l.point(ptab, e), l.point(ptab, e + 1));
+          const uint2 y = make_uint2(l.point(ptab, e + 2), l.point(ptab, e + 3));
+          list[p] = x;
+          list[p + 1] = y;
+          dst[p] = sl;
+          dst[p + 1] = sl + 1;
+        }
+        if (i < pairs) {
+          list[p] = make_uint2(l.point(ptab, e), l.point(ptab, e + 1));
+          dst[p++] = sl++;
+          e += 2;
+        }
+      }
+      if (r.n[s] & 1) {
+        const uint32_t v = l.point(ptab, e);
+        G1Aff q = ld_aff(tab + (v & 0x7fffffffu));
+        if (v >> 31) q.y = -q.y;
+        st_aff(slots + sl++, q);
+      }
+    }
+  }
+  if (threadIdx.x == FB_ACC_THREADS - 1) sh.sstart[k0 + per] = (uint16_t)sl;
+  return total & 0xffffu;
+}
+// the later levels: slots 2^lst apart of each bucket
+static __device__ __noinline__ uint32_t bkt_list_next(BktShared& sh, uint32_t k0, uint32_t per, uint32_t lst,
+                                                      uint32_t* dst) {
+  if (threadIdx.x == 0) sh.runs = 0;
+  auto pairs_of = [&](uint32_t k) {
+    return ((uint32_t)sh.sstart[k + 1] - sh.sstart[k] + (1u << lst) - 1) >> (lst + 1);
+  };
+  uint32_t cnt = 0, np;
+  for (uint32_t k = k0; k < k0 + per; ++k) cnt += pairs_of(k);
+  uint32_t p = block_scan(cnt, sh.wsum, &np);
+  for (uint32_t k = k0; k < k0 + per; ++k) {
+    const uint32_t s0 = sh.sstart[k], pairs = pairs_of(k);
+    if (pairs >= FB_RUN_PAIRS && sh.defer(s0, 0, pairs, p, 0)) p += pairs;
+    else
+      for (uint32_t i = 0; i < pairs; ++i) dst[p++] = s0 + (i << (lst + 1));
+  }
+  return np;
+}
+// the runs that bkt_list_first left to the CTA
+template <class U>
+static __device__ __noinline__ void bkt_runs_first(const BktShared& sh, const BktLists<U> l, uint2* list,
+                                                   uint32_t* dst) {
+  const uint32_t runs = min(sh.runs, FB_RUNS_MAX);
+  for (uint32_t r = 0; r < runs; ++r) {
+    const uint4 q = sh.run[r];
+    const uint32_t p = q.w & 0xffffu;
+    for (uint32_t i = threadIdx.x; i < q.z; i += FB_ACC_THREADS) {
+      list[p + i] = make_uint2(l.point(q.y, q.x + 2 * i), l.point(q.y, q.x + 2 * i + 1));
+      dst[p + i] = (q.w >> 16) + i;
+    }
+  }
+}
+// the runs that bkt_list_next left to the CTA
+static __device__ __noinline__ void bkt_runs_next(const BktShared& sh, uint32_t lst, uint32_t* dst) {
+  const uint32_t runs = min(sh.runs, FB_RUNS_MAX);
+  for (uint32_t r = 0; r < runs; ++r) {
+    const uint4 q = sh.run[r];
+    for (uint32_t i = threadIdx.x; i < q.z; i += FB_ACC_THREADS) dst[(q.w & 0xffffu) + i] = q.x + (i << (lst + 1));
+  }
+}
+
 // One addition of a level: what its list entry says (read ahead), and where
 // its points are
 struct BktDesc {
@@ -406,12 +571,10 @@ template <class M>
 __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     k_fb_accum(const FbAccPlan plan, const FbScratch scratch, uint32_t* __restrict__ next, uint32_t task) {
   constexpr uint32_t T = FB_ACC_THREADS;
-  constexpr uint32_t NB = FB_GROUP * FB_BUCKETS;
   __shared__ uint4 stg[10][T];           // the passes' staging rows
   __shared__ Fq sp[T];
-  __shared__ uint16_t sstart[NB + 1];    // first slot of each bucket
+  __shared__ BktShared sh;
   __shared__ uint32_t first[FB_GROUP + 1];  // entries before each item of the group
-  __shared__ uint32_t wsum[T / 32];
   __shared__ uint32_t item;
   const uint32_t tid = threadIdx.x;
   uint8_t* const mem = scratch.base + (size_t)blockIdx.x * scratch.bytes();
@@ -441,54 +604,40 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     const FbAccArgs& a = plan.a[set];
     const uint32_t ng = (plan.start[set + 1] - plan.start[set] - u0 + groups - 1) / groups;
     const bool wide = a.ents32 != nullptr;
-    // item i of the group: its bucket offsets, entries and first table point
-    struct Item {
-      const uint32_t *offs, *offs2;
-      const void *ents, *ents2;
-      uint32_t tab;
-    };
+    const BktLists<uint32_t> lists32{a.ents32, (uint32_t)a.ulog, (uint32_t)a.tabN};
+    const BktLists<uint16_t> lists16{a.ents, 10u, (uint32_t)a.tabN};
+    // item i of the group
     auto item_of = [&](uint32_t i) {
       const uint32_t u = u0 + i * groups, nch = 1u << a.lr;
       const uint32_t l = u % a.lines, g = u / a.lines;
       const uint32_t coset = g / nch, b = g % nch;
-      Item it;
+      BktItem it;
       it.offs2 = nullptr;
-      it.ents2 = nullptr;
+      it.ents2 = 0;
       it.tab = (coset * a.Ltot + a.l0 + l) * a.W * (uint32_t)a.tabN;
       if (wide) {
         const int bl = a.ulog - 10, ml = a.mlog;
         const uint32_t unit = b >> bl, blk = b & ((1u << bl) - 1);
-        const size_t cu = (size_t)coset * ((size_t)(nch >> bl) << ml) + ((size_t)unit << ml);  // first sort unit
-        it.offs = a.offs + cu * ((1u << a.ulog) + 1) + (size_t)blk * FB_BUCKETS;
-        it.ents = a.ents32 + cu * wd_unit_ents(a.ulog);
+        const uint32_t cu = coset * ((nch >> bl) << ml) + (unit << ml);  // first sort unit
+        it.offs = a.offs + (size_t)cu * ((1u << a.ulog) + 1) + (size_t)blk * FB_BUCKETS;
+        it.ents = cu * (uint32_t)wd_unit_ents(a.ulog);
         if (ml) {
           it.offs2 = it.offs + ((1u << a.ulog) + 1);
-          it.ents2 = a.ents32 + (cu + 1) * wd_unit_ents(a.ulog);
+          it.ents2 = it.ents + (uint32_t)wd_unit_ents(a.ulog);
         }
         it.tab += unit << (a.ulog + ml);
       } else {
         it.offs = a.offs + (size_t)g * (FB_BUCKETS + 1);
-        it.ents = a.ents + (size_t)g * FB_WINDOWS * (1u << a.lc);
+        it.ents = g * (FB_WINDOWS << a.lc);
         it.tab += b << a.lc;
       }
       return it;
-    };
-    // table point (from a.tab) and sign bit of entry e of an item's sort unit 0 or 1
-    auto entry = [&](const Item& it, int second, uint32_t e) -> uint32_t {
-      const uint32_t N = (uint32_t)a.tabN;
-      if (wide) {
-        const uint32_t v = reinterpret_cast<const uint32_t*>(second ? it.ents2 : it.ents)[e], lg = (uint32_t)a.ulog;
-        const uint32_t idx = (v & ((1u << lg) - 1)) + (second ? 1u << lg : 0u);
-        return (it.tab + ((v >> lg) & 31) * N + idx) | (v & 0x80000000u);
-      }
-      const uint32_t v = reinterpret_cast<const uint16_t*>(it.ents)[e];
-      return (it.tab + ((v >> 10) & 31) * N + (v & 0x3ff)) | ((v & 0x8000u) << 16);
     };
     if (tid == 0) {
       uint32_t n = 0;
       for (uint32_t i = 0; i < ng; ++i) {
         first[i] = n;
-        const Item it = item_of(i);
+        const BktItem it = item_of(i);
         n += it.offs[FB_BUCKETS] - it.offs[0];
         if (it.offs2) n += it.offs2[FB_BUCKETS] - it.offs2[0];
       }
@@ -498,74 +647,21 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
     const uint32_t nent = first[ng];
     // this thread's buckets k0 .. k0 + per - 1 are item my's
     const uint32_t per = (ng <= 2 ? ng : 4) * (FB_BUCKETS / T), k0 = tid * per, my = k0 / FB_BUCKETS;
-    uint32_t seg = 0, st = 0, h = 0, lh = 0;
-    int mode = 0;  // 0: level 1 of segment seg, 1: slots st apart, 2: grid level of half width h
+    uint32_t seg = 0, st = 0, lst = 0, h = 0, lh = 0;
+    int mode = 0;  // 0: level 1 of segment seg, 1: slots 2^lst apart, 2: grid level of half width h
     for (;;) {
       uint32_t np = 0;
       if (mode == 0) {
-        const uint32_t lo = seg * cap, hi = min(nent, lo + cap);
-        Item it = item_of(min(my, ng - 1));
-        const uint32_t f0 = it.offs[0], f1 = it.offs2 ? it.offs2[0] : 0u;
-        // the range of the segment in bucket k (of item my), as entry ranges of its two sort units
-        struct Part {
-          uint32_t e[2], n[2], carry;
-        };
-        auto part = [&](uint32_t k) {
-          Part p = {};
-          if (my >= ng) return p;
-          const uint32_t b = k % FB_BUCKETS;
-          const uint32_t o0 = it.offs[b], c0 = it.offs[b + 1] - o0;
-          const uint32_t o1 = it.offs2 ? it.offs2[b] : 0u, c1 = it.offs2 ? it.offs2[b + 1] - o1 : 0u;
-          const uint32_t at = first[my] + (o0 - f0) + (o1 - f1);
-          const uint32_t qa = min(max(lo, at) - at, c0 + c1), qb = hi > at ? max(qa, min(hi - at, c0 + c1)) : qa;
-          const uint32_t a0 = min(qa, c0), b0 = min(qb, c0);
-          p.e[0] = o0 + a0;
-          p.n[0] = b0 - a0;
-          p.e[1] = o1 + (qa - a0);
-          p.n[1] = (qb - b0) - (qa - a0);
-          p.carry = at < lo && qb > qa;  // the bucket began in an earlier segment
-          return p;
-        };
-        uint32_t cnt = 0;  // pairs | slots << 16
-        for (uint32_t k = k0; k < k0 + per; ++k) {
-          const Part p = part(k);
-          cnt += ((p.n[0] >> 1) + (p.n[1] >> 1)) + ((((p.n[0] + 1) >> 1) + ((p.n[1] + 1) >> 1) + p.carry) << 16);
-        }
-        uint32_t total;
-        const uint32_t at = block_scan(cnt, wsum, &total);
-        uint32_t p = at & 0xffffu, sl = at >> 16;
-        np = total & 0xffffu;
-        for (uint32_t k = k0; k < k0 + per; ++k) {
-          const Part r = part(k);
-          sstart[k] = (uint16_t)sl;
-          if (r.carry) st_aff(slots + sl++, ld_aff(fin + k));
-#pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint32_t end = r.e[s] + r.n[s];
-            for (uint32_t e = r.e[s]; e + 1 < end; e += 2) {
-              list[p] = make_uint2(entry(it, s, e), entry(it, s, e + 1));
-              dst[p++] = sl++;
-            }
-            if (r.n[s] & 1) {
-              const uint32_t v = entry(it, s, end - 1);
-              G1Aff q = ld_aff(a.tab + (v & 0x7fffffffu));
-              if (v >> 31) q.y = -q.y;
-              st_aff(slots + sl++, q);
-            }
-          }
-        }
-        if (tid == T - 1) sstart[k0 + per] = (uint16_t)sl;
+        const uint32_t lo = seg * cap, mine = min(my, ng - 1);
+        const BktItem it = item_of(mine);
+        const uint32_t hi = min(nent, lo + cap);
+        np = wide ? bkt_list_first(sh, lists32, it, my < ng, first[mine], lo, hi, k0, per, a.tab, slots, fin, list, dst)
+                  : bkt_list_first(sh, lists16, it, my < ng, first[mine], lo, hi, k0, per, a.tab, slots, fin, list, dst);
       } else if (mode == 1) {
-        uint32_t cnt = 0;
-        for (uint32_t k = k0; k < k0 + per; ++k) cnt += ((uint32_t)sstart[k + 1] - sstart[k] + st - 1) / st >> 1;
-        uint32_t p = block_scan(cnt, wsum, &np);
-        for (uint32_t k = k0; k < k0 + per; ++k) {
-          const uint32_t s0 = sstart[k], pairs = ((uint32_t)sstart[k + 1] - s0 + st - 1) / st >> 1;
-          for (uint32_t i = 0; i < pairs; ++i) dst[p++] = s0 + 2 * i * st;
-        }
+        np = bkt_list_next(sh, k0, per, lst, dst);
         if (np == 0) {  // one sum per bucket left
           for (uint32_t k = tid; k < ng * FB_BUCKETS; k += T) {
-            if (sstart[k + 1] > sstart[k]) st_aff(fin + k, ld_aff(slots + sstart[k]));
+            if (sh.sstart[k + 1] > sh.sstart[k]) st_aff(fin + k, ld_aff(slots + sh.sstart[k]));
             else if (seg == 0) st_aff(fin + k, aff_inf());
           }
           ++seg;
@@ -583,6 +679,12 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
         np = ng * FB_OUT * h;
       }
       __syncthreads();
+      if (sh.runs) {  // the same for all threads; 0 in grid levels
+        if (mode != 0) bkt_runs_next(sh, lst, dst);
+        else if (wide) bkt_runs_first(sh, lists32, list, dst);
+        else bkt_runs_first(sh, lists16, list, dst);
+        __syncthreads();
+      }
       const uint32_t lmode = (uint32_t)mode;
       auto fetch = [&](uint32_t j, bool there) {
         BktDesc c = {0, 0, 0};
@@ -628,8 +730,10 @@ __global__ void __launch_bounds__(FB_ACC_THREADS, FB_ACC_MIN_CTAS)
       if (mode == 0) {
         mode = 1;
         st = 1;
+        lst = 0;
       } else if (mode == 1) {
         st *= 2;
+        ++lst;
       } else {
         if (h == 1) break;
         h >>= 1;
