@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/zg_encoder.h"
+#include "zg_host.hpp"
 #include "zg_kernels.cuh"
 #include "zg_recover.cuh"
 #include "zg_verify.cuh"
@@ -405,50 +406,6 @@ void pinned_put(void* p, size_t bytes) {
   } else {
     cudaFreeHost(p);
   }
-}
-}  // namespace
-
-// Runs fn(i) for i < n on up to 16 host threads, `grain` indexes at a time (the
-// caller's thread alone when there is one grain or threads cannot be had).
-// false if a call threw (out of memory); the other indexes still run.
-namespace {
-template <class F>
-bool host_parallel(size_t n, size_t grain, F fn) {
-  std::atomic<size_t> next{0};
-  std::atomic<bool> ok{true};
-  auto work = [&] {
-    for (size_t b; (b = next.fetch_add(grain)) < n;)
-      for (size_t i = b; i < std::min(n, b + grain); ++i) {
-        try {
-          fn(i);
-        } catch (...) {
-          ok = false;
-        }
-      }
-  };
-  const size_t blocks = (n + grain - 1) / grain;
-  const size_t want = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()), blocks});
-  std::vector<std::thread> more;
-  try {
-    more.reserve(want);
-    for (size_t t = 1; t < want; ++t) more.emplace_back(work);
-  } catch (...) {
-  }
-  work();
-  for (std::thread& t : more) t.join();
-  return ok;
-}
-// memcpy, by several threads from 4 MiB on: one thread moves some 8 GB/s
-// between pageable and pinned memory, a blob's rows are 50 MB
-void host_copy(void* dst, const void* src, size_t n) {
-  constexpr size_t kPart = 1 << 20;
-  if (n < 4 * kPart) {
-    memcpy(dst, src, n);
-    return;
-  }
-  host_parallel((n + kPart - 1) / kPart, 1, [&](size_t i) {
-    memcpy((uint8_t*)dst + i * kPart, (const uint8_t*)src + i * kPart, std::min(kPart, n - i * kPart));
-  });
 }
 }  // namespace
 
@@ -2924,7 +2881,7 @@ int zg_verify_slices(zg_ctx* c, const uint8_t* const* slices, const size_t* lens
   // the deserialization on the host's threads (22 on-curve checks and 1024
   // range checks per production slice)
   std::vector<uint8_t> parsed(n, 0);
-  if (!host_parallel(n, 8, [&](size_t i) {
+  if (!host_parallel(n, 8, 16, [&](size_t i) {
         parsed[i] = auth_ok && slices[i] && parse_slice(slices[i], lens[i], &sl[i]);
       }))
     return fail(ZG_ERR_INTERNAL, "verify: out of host memory");
@@ -2963,7 +2920,7 @@ int zg_verify_slices(zg_ctx* c, const uint8_t* const* slices, const size_t* lens
       v.dpos[i] = (uint32_t)j;
       nproof[j] = (uint32_t)sl[i].nmerkle;
     }
-    host_parallel(nb, 8, [&](size_t j) { memcpy(stage + j * v.stride, slices[batch[j]], lens[batch[j]]); });
+    host_copies(nb, v.stride, [&](size_t j) { memcpy(stage + j * v.stride, slices[batch[j]], lens[batch[j]]); });
     v.d_slices = v.dev<uint8_t>(nb * v.stride);
     v.d_scal = v.dev<uint8_t>(3 * c->N * 32);
     uint32_t* d_np = v.dev<uint32_t>(nb);
@@ -3339,8 +3296,7 @@ int zg_recover(zg_ctx* c, const uint64_t* row_ids, const uint8_t* const* rows, c
     known[4 * r + (cs == 1 ? 2 : (cs == 2 ? 1 : cs))] = 1;
     ++k;
   }
-  host_parallel(k, std::max<size_t>(1, (1 << 18) / (32 * C)),
-                [&](size_t i) { memcpy(c->h_rec + i * 32 * C, from[i], 32 * C); });
+  host_copies(k, 32 * C, [&](size_t i) { memcpy(c->h_rec + i * 32 * C, from[i], 32 * C); });
   std::vector<uint16_t> erased;
   for (size_t i = 0; i < M; ++i)
     if (!known[i]) erased.push_back((uint16_t)i);
