@@ -108,9 +108,12 @@ struct Twiddles {
   Fr *twf_c = nullptr, *twi_c = nullptr, *twf_r = nullptr, *twi_r = nullptr;
   Fr *wn_lo = nullptr, *wn_hi = nullptr, *wni_lo = nullptr, *wni_hi = nullptr;
   Fr *gs_lo = nullptr, *gs_hi = nullptr;  // coset scale tables (cosets 1, 2)
-  // the column pass's factors in its own order, [column][row], for zg_ntt:
-  // w_N^(s r) and w_N^(-s r) / N
+  // zg_ntt's (cached_twiddles): wni_lo / N, and the column pass's factors in its
+  // own order, [column][row]: w_N^(s r) and w_N^(-s r) / N (null before the first
+  // use, and for good once that found no room)
+  Fr* wni_lo_n = nullptr;
   Fr *wn_full = nullptr, *wni_full = nullptr;
+  bool full_asked[2] = {false, false};
 };
 
 template <class T>
@@ -167,7 +170,7 @@ int make_twiddles(int lr, int lc, Twiddles* tw) {
 }
 void free_twiddles(Twiddles* tw) {
   Fr* ps[] = {tw->twf_c, tw->twi_c, tw->twf_r, tw->twi_r, tw->wn_lo, tw->wn_hi,
-              tw->wni_lo, tw->wni_hi, tw->gs_lo, tw->gs_hi, tw->wn_full, tw->wni_full};
+              tw->wni_lo, tw->wni_hi, tw->gs_lo, tw->gs_hi, tw->wni_lo_n, tw->wn_full, tw->wni_full};
   for (Fr* p : ps) if (p) cudaFree(p);
   *tw = Twiddles();
 }
@@ -199,7 +202,8 @@ int set_smem_limits() {
   ZG_CK(cudaFuncSetAttribute(k_msm_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_fb_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_wd_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  ZG_CK(cudaFuncSetAttribute(k_ntt4_colpass, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  ZG_CK(cudaFuncSetAttribute(k_ntt4_colpass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  ZG_CK(cudaFuncSetAttribute(k_ntt4_colpass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   ZG_CK(cudaFuncSetAttribute(k_ntt4_rowpass, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   done.insert(dev);
   return 0;
@@ -215,19 +219,19 @@ inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t);
 // one inverse of 2^20 209, 230 and 280 us.
 unsigned ntt_threads(int logn) { return (unsigned)std::min(256, std::max(32, 1 << std::max(0, logn - 2))); }
 
-// natural-order N-point transform out = DFT(x) (or inverse without 1/N), via
-// the column / row passes; tmp has N elements
+// natural-order N-point transform out = DFT(x) (or inverse, without 1/N unless
+// `scaled`), via the column / row passes; tmp has N elements
 // (batch vectors back to back in x, tmp and out; batch <= 65535). With cs
-// set, input q C + s of each vector is first multiplied by cs[s R + q] (coset
-// shift). wfull: w_N^(+-s r) in the column pass's order, scale included, or
-// null (products of the two power tables).
+// set, input q C + s of each vector is first multiplied by cs[s R + q], or by
+// cs[s] cs_hi[q] (coset shift). wfull: w_N^(+-s r) in the column pass's order,
+// scale included, or null (products of the two power tables).
 void ntt4(const Twiddles& tw, const Fr* x, Fr* tmp, Fr* out, bool inverse, cudaStream_t s, uint32_t batch = 1,
-          const Fr* wfull = nullptr, const Fr* cs = nullptr) {
+          bool scaled = false, const Fr* wfull = nullptr, const Fr* cs = nullptr, const Fr* cs_hi = nullptr) {
   const int lr = tw.lr, lc = tw.lc;
   const size_t R = size_t(1) << lr, C = size_t(1) << lc;
-  k_ntt4_colpass<<<dim3((unsigned)C, batch), ntt_threads(lr), R * sizeof(Fr), s>>>(
-      x, tmp, lr, lc, inverse ? tw.twi_r : tw.twf_r, inverse ? tw.wni_lo : tw.wn_lo, inverse ? tw.wni_hi : tw.wn_hi,
-      wfull, cs);
+  const Fr* w_lo = inverse ? (scaled ? tw.wni_lo_n : tw.wni_lo) : tw.wn_lo;
+  (cs_hi ? k_ntt4_colpass<true> : k_ntt4_colpass<false>)<<<dim3((unsigned)C, batch), ntt_threads(lr), R * sizeof(Fr), s>>>(
+      x, tmp, lr, lc, inverse ? tw.twi_r : tw.twf_r, w_lo, inverse ? tw.wni_hi : tw.wn_hi, wfull, cs, cs_hi);
   k_ntt4_rowpass<<<dim3((unsigned)R, batch), ntt_threads(lc), C * sizeof(Fr), s>>>(
       tmp, out, lr, lc, inverse ? tw.twi_c : tw.twf_c);
 }
@@ -1288,72 +1292,99 @@ const Twiddles* cached_twiddles(int lr, int lc) {
   if (it != g_ntt_tw.end()) return &it->second;
   Twiddles t;
   if (make_twiddles(lr, lc, &t)) return nullptr;
+  if (lr) {
+    const Fr ninv = host_fr_from_u32(1u << (lr + lc)).inverse();
+    std::vector<Fr> lo = pow_table(fr_root(lr + lc).inverse(), size_t(1) << lc);
+    for (Fr& x : lo) x = x * ninv;
+    if (upload(&t.wni_lo_n, lo)) return nullptr;
+  }
   return &(g_ntt_tw[key] = t);
 }
 
-// Factor tables of the standalone transforms, built on the device on their
-// first use and kept for the process: out[s R + r] = base^(s r) scale
-// (`shift` false) or base^(r C + s) (true), from the split power tables lo[C]
-// and hi[R] of base.
-int build_full_table(const Fr* lo, const Fr* hi, int lr, int lc, bool shift, const Fr& scale, Fr** out) {
-  const size_t N = size_t(1) << (lr + lc);
+// Full factor tables of the standalone transforms above 2^11 points, built on
+// the device on their first use and kept for the process (captured graphs hold
+// their addresses): 32 bytes a point for each direction and coset, up to
+// FULL_TABLES_MAX a device in all. A transform that finds no room, in that sum
+// or in the device memory, goes on with the split power tables, two products
+// more per element of a coset transform and one of the others (one inverse of
+// 2^20 247 against 209 us).
+constexpr size_t FULL_TABLES_MAX = size_t(256) << 20;
+std::map<int, size_t> g_full_bytes;  // per device; guarded by g_ntt_mu
+
+// out[s R + r] = base^(s r) scale (`shift` false) or base^(r C + s) (true), from
+// the split power tables lo[C] and hi[R] of base; null when there is no room.
+// The build has a stream of its own and ends before it returns, so it may come
+// while the caller's stream, or another thread's, is being captured.
+Fr* build_full_table(const Fr* lo, const Fr* hi, int lr, int lc, bool shift, const Fr& scale) {
+  const size_t N = size_t(1) << (lr + lc), bytes = N * sizeof(Fr);
+  size_t& held = g_full_bytes[current_device()];
+  if (held + bytes > FULL_TABLES_MAX) return nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   Fr* t = nullptr;
-  ZG_CK(cudaMalloc(&t, N * sizeof(Fr)));
   cudaStream_t s = nullptr;
-  bool ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  bool ok = cudaMalloc(&t, bytes) == cudaSuccess && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
   if (ok) {
     k_full_table<<<nblk(N, 256), 256, 0, s>>>(lo, hi, lr, lc, shift ? 1 : 0, scale, t);
     ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
-    cudaStreamDestroy(s);
   }
+  if (s) cudaStreamDestroy(s);
   if (!ok) {
-    cudaFree(t);
-    return fail(ZG_ERR_CUDA, "transform table build failed");
+    if (t) cudaFree(t);
+    t = nullptr;
+    cudaGetLastError();
   }
-  *out = t;
-  return 0;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (ok) held += bytes;
+  return t;
 }
 
 // the coset factors g^i of zg_ntt per (device, logn, coset): i < 2^logn in
-// order up to the single-CTA transform's size, in the column pass's order
-// above it
-std::map<std::tuple<int, int, uint32_t>, Fr*> g_coset_pows;  // guarded by g_ntt_mu
+// order up to the single-CTA transform's size (lo); above it in the column
+// pass's order (lo), or split, lo[i mod C] hi[i / C]
+struct CosetPows {
+  Fr* lo = nullptr;
+  Fr* hi = nullptr;
+};
+std::map<std::tuple<int, int, uint32_t>, CosetPows> g_coset_pows;  // guarded by g_ntt_mu
 
-const Fr* cached_coset_pows(int logn, uint32_t coset) {
+const CosetPows* cached_coset_pows(int logn, uint32_t coset) {
   std::lock_guard<std::mutex> g(g_ntt_mu);
   auto key = std::make_tuple(current_device(), logn, coset);
   auto it = g_coset_pows.find(key);
-  if (it != g_coset_pows.end()) return it->second;
+  if (it != g_coset_pows.end()) return &it->second;
   const Fr gen = coset_factor(logn, coset);
-  Fr* t = nullptr;
+  CosetPows p;
   if (logn <= 11) {
-    if (upload(&t, pow_table(gen, size_t(1) << logn))) return nullptr;
+    if (upload(&p.lo, pow_table(gen, size_t(1) << logn))) return nullptr;
   } else {
     const int lc = (logn + 1) / 2, lr = logn - lc;
-    Fr *lo = nullptr, *hi = nullptr;
-    int rc = upload(&lo, pow_table(gen, size_t(1) << lc));
-    if (!rc) rc = upload(&hi, pow_table(gen.pow_u64(uint64_t(1) << lc), size_t(1) << lr));
-    if (!rc) rc = build_full_table(lo, hi, lr, lc, true, Fr::one(), &t);
-    if (lo) cudaFree(lo);
-    if (hi) cudaFree(hi);
-    if (rc) return nullptr;
+    if (upload(&p.lo, pow_table(gen, size_t(1) << lc)) ||
+        upload(&p.hi, pow_table(gen.pow_u64(uint64_t(1) << lc), size_t(1) << lr))) {
+      if (p.lo) cudaFree(p.lo);
+      return nullptr;
+    }
+    if (Fr* full = build_full_table(p.lo, p.hi, lr, lc, true, Fr::one())) {
+      cudaFree(p.lo);
+      cudaFree(p.hi);
+      p = CosetPows{full, nullptr};
+    }
   }
-  return g_coset_pows[key] = t;
+  return &(g_coset_pows[key] = p);
 }
 
 // the column pass's factors of a transform of zg_ntt (with 1/N for the
-// inverse), one direction at a time; null on failure
+// inverse), one direction at a time, or null
 const Fr* cached_full_twiddles(const Twiddles* tw, bool inverse) {
   std::lock_guard<std::mutex> g(g_ntt_mu);
   Twiddles* t = const_cast<Twiddles*>(tw);  // an entry of g_ntt_tw
-  Fr** full = inverse ? &t->wni_full : &t->wn_full;
-  if (!*full) {
-    const Fr ninv = host_fr_from_u32(1u << (tw->lr + tw->lc)).inverse();
-    if (build_full_table(inverse ? tw->wni_lo : tw->wn_lo, inverse ? tw->wni_hi : tw->wn_hi, tw->lr, tw->lc, false,
-                         inverse ? ninv : Fr::one(), full))
-      return nullptr;
+  if (!t->full_asked[inverse]) {
+    t->full_asked[inverse] = true;
+    const Fr* lo = inverse ? tw->wni_lo_n : tw->wn_lo;
+    (inverse ? t->wni_full : t->wn_full) =
+        build_full_table(lo, inverse ? tw->wni_hi : tw->wn_hi, tw->lr, tw->lc, false, Fr::one());
   }
-  return *full;
+  return inverse ? t->wni_full : t->wn_full;
 }
 
 // The stream-ordered pool of the current device keeps freed memory instead of
@@ -3487,8 +3518,12 @@ int zg_ntt(void* d_data, uint32_t log_n, uint32_t batch, int inverse, uint32_t c
   ZG_CK(cudaFuncSetAttribute(k_ntt_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   const size_t n = size_t(1) << log_n;
   Fr* v = (Fr*)d_data;
-  const Fr* cs = nullptr;
-  if (coset_idx && !(cs = cached_coset_pows((int)log_n, coset_idx))) return fail(ZG_ERR_CUDA, "coset table alloc failed");
+  CosetPows cs;
+  if (coset_idx) {
+    const CosetPows* p = cached_coset_pows((int)log_n, coset_idx);
+    if (!p) return fail(ZG_ERR_CUDA, "coset table alloc failed");
+    cs = *p;
+  }
   // the transforms run on the canonical values directly (linear passes with
   // Montgomery-form twiddles keep canonical values canonical); the coset
   // shift is a product of the transforms' first loads, the inverse's 1/n part
@@ -3500,22 +3535,21 @@ int zg_ntt(void* d_data, uint32_t log_n, uint32_t batch, int inverse, uint32_t c
     for (uint32_t b0 = 0; b0 < batch;) {
       uint32_t nb = std::min<uint32_t>(batch - b0, 65535);
       k_ntt_small<<<nb, ntt_threads((int)log_n), n * sizeof(Fr), s>>>(
-          v + (size_t)b0 * n, (int)log_n, inverse ? tw->twi_c : tw->twf_c, cs, inverse, ninv);
+          v + (size_t)b0 * n, (int)log_n, inverse ? tw->twi_c : tw->twf_c, cs.lo, inverse, ninv);
       b0 += nb;
     }
   } else {
     const int lc = (int)(log_n + 1) / 2, lr = (int)log_n - lc;
     const Twiddles* tw = cached_twiddles(lr, lc);
     if (!tw) return ZG_ERR_CUDA;
-    const Fr* wfull = cached_full_twiddles(tw, inverse != 0);
-    if (!wfull) return ZG_ERR_CUDA;
+    const Fr* wfull = cached_full_twiddles(tw, inverse != 0);  // or null
     const uint32_t per = std::min<uint32_t>(batch, 65535);
     keep_pool_memory();
     Fr* tmp = nullptr;
     ZG_CK(cudaMallocAsync(&tmp, (size_t)per * n * sizeof(Fr), s));
     for (uint32_t b0 = 0; b0 < batch; b0 += per) {
       const uint32_t nb = std::min<uint32_t>(batch - b0, per);
-      ntt4(*tw, v + (size_t)b0 * n, tmp, v + (size_t)b0 * n, inverse != 0, s, nb, wfull, cs);
+      ntt4(*tw, v + (size_t)b0 * n, tmp, v + (size_t)b0 * n, inverse != 0, s, nb, true, wfull, cs.lo, cs.hi);
     }
     cudaFreeAsync(tmp, s);
   }

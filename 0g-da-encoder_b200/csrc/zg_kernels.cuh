@@ -1470,18 +1470,20 @@ __global__ void __launch_bounds__(256) k_full_table(const Fr* __restrict__ lo, c
 // generic four-step NTT pass A: for each column s (C of them) of x viewed as
 // [R][C] row-major: R-point transform over q, times w_N^{s r}; writes Y[r][s].
 // blockIdx.y selects the vector of a batch (vectors of R C elements back to back).
-// With cs set, element q C + s of x is first multiplied by cs[s R + q] (the
-// coset shift); with wfull set the factors w_N^{s r} (and a scale) are
+// With cs set, element q C + s of x is first multiplied by cs[s R + q] or
+// (SPLIT, an instance of its own: with both in one kernel the inverse of 2^20 took
+// 225 us) by cs[s] cs_hi[q] (the coset shift); with wfull set the factors w_N^{s r} (and a scale) are
 // wfull[s R + r], read in order by the CTA of column s, else products of the
 // split tables. Bound by the field products (N (log2 N) / 2 of them and one per
 // factor); the full tables take two products per element of a coset transform
 // away (the power w_N^{s r} and the coset's lo hi) and the 1/N product of the
 // last stores: 64 coset transforms of 2^14 207 -> 159 us, one inverse of 2^20
 // 247 -> 209 us, 20% and 33% above the products' own time.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_ntt4_colpass(const Fr* __restrict__ x, Fr* __restrict__ y, int lr, int lc,
                                const Fr* __restrict__ tw_r, const Fr* __restrict__ w_lo,
                                const Fr* __restrict__ w_hi, const Fr* __restrict__ wfull,
-                               const Fr* __restrict__ cs) {
+                               const Fr* __restrict__ cs, const Fr* __restrict__ cs_hi) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int C = 1 << lc;
   Fr* s = reinterpret_cast<Fr*>(smem);
@@ -1491,6 +1493,7 @@ __global__ void __launch_bounds__(256) k_ntt4_colpass(const Fr* __restrict__ x, 
   const uint32_t nmask = (1u << (lr + lc)) - 1;
   auto get = [&](int q) {
     const Fr e = load_fr(x + (size_t)q * C + col);
+    if (SPLIT) return e * (cs[col] * cs_hi[q]);
     return cs ? e * load_fr(cs + ((size_t)col << lr) + q) : e;
   };
   ntt_block(s, lr, tw_r, get, [&](int r, const Fr& v) { s[r] = v; });

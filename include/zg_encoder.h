@@ -347,7 +347,13 @@ int zg_msm_chunks_noalloc(const void* d_bases, const void* d_scalars, uint32_t l
  * (crates/amt/src/blob/encode.rs:142-157): `batch` contiguous vectors of
  * 2^log_n canonical 32-byte elements, transformed in place. inverse != 0
  * applies the 1/n scaled inverse. coset_idx > 0 (forward only) multiplies
- * coefficient i by coset_factor(2^log_n, coset_idx)^i first (to_coset_blob). */
+ * coefficient i by coset_factor(2^log_n, coset_idx)^i first (to_coset_blob).
+ * The first call of a size, direction or coset on a device builds factor tables
+ * and waits for them: make the first call of a size and coset before a stream
+ * capture (its other direction may come first inside one). The tables stay for
+ * the process, at most 256 MiB a device above 2^11 points (32 bytes a point,
+ * direction and coset; sizes beyond that run on smaller tables, some 20 %
+ * slower). */
 int zg_ntt(void* d_data, uint32_t log_n, uint32_t batch, int inverse, uint32_t coset_idx, void* stream);
 /* Keccak-256 Merkle levels (crates/encoder/src/merkle/blob.rs:15-34) over
  * n_items 32-byte items: leaves = keccak(8 items), then pairwise parents
