@@ -84,27 +84,40 @@ constexpr int FB_GROUP = 4;
 // 126 ms. Lines of 32 to 160 pairs time alike.
 constexpr uint32_t FB_RUN_PAIRS = 64;
 constexpr uint32_t FB_RUNS_MAX = 192;
-// Per-CTA scratch, for segments of at most `cap` entries.
+// Scratch of `ctas` CTAs, for turns of up to `group` items and segments of at
+// most `cap` entries, in five blocks (GAP bytes that nothing touches after each).
 struct FbScratch {
   uint8_t* base = nullptr;
   uint32_t cap = 0;
-  // level-1 sums of a segment: half its entries, two odd ones and a carried
-  // sum per bucket
-  __host__ __device__ uint32_t slots() const { return cap / 2 + 3 * FB_GROUP * FB_BUCKETS; }
-  __host__ __device__ size_t off_fin() const { return (size_t)slots() * sizeof(G1Aff); }
-  __host__ __device__ size_t off_pre() const { return off_fin() + FB_GROUP * FB_BUCKETS * sizeof(G1Aff); }
-  __host__ __device__ size_t off_list() const {
-    return off_pre() + (size_t)fb_batch(FB_TASK_MAX) * FB_ACC_THREADS * sizeof(Fq);
+  uint32_t group = FB_GROUP;
+  uint32_t ctas = 0;
+  static constexpr size_t GAP = 16;
+  // level-1 sums of a segment: half its entries, an odd one per bucket and sort
+  // unit (half a slot each), and a carried sum
+  __host__ __device__ uint32_t slots() const { return cap / 2 + group * FB_BUCKETS + 1; }
+  // additions per thread and batch: of the longest level (level 1, or the grid's
+  // FB_BUCKETS per item)
+  __host__ __device__ uint32_t batch() const {
+    const uint32_t most = (max2(cap / 2, group * FB_BUCKETS) + FB_ACC_THREADS - 1) / FB_ACC_THREADS;
+    return most < fb_batch(FB_TASK_MAX) ? most : fb_batch(FB_TASK_MAX);
   }
-  __host__ __device__ size_t off_dst() const { return off_list() + (size_t)(cap / 2) * sizeof(uint2); }
+  __host__ __device__ size_t off_fin() const { return after(0, (size_t)slots() * sizeof(G1Aff)); }
+  __host__ __device__ size_t off_pre() const { return after(off_fin(), (size_t)group * FB_BUCKETS * sizeof(G1Aff)); }
+  __host__ __device__ size_t off_list() const { return after(off_pre(), (size_t)batch() * FB_ACC_THREADS * sizeof(Fq)); }
+  __host__ __device__ size_t off_dst() const { return after(off_list(), (size_t)(cap / 2) * sizeof(uint2)); }
+  // a bucket's slots pair up to at most half of the segment's entries and carry
   __host__ __device__ size_t bytes() const {
-    return (off_dst() + ((size_t)cap / 2 + 16) * sizeof(uint32_t) + 255) / 256 * 256;
+    return (after(off_dst(), ((size_t)cap / 2 + 1) * sizeof(uint32_t)) + 255) / 256 * 256;
   }
+
+ private:
+  __host__ __device__ static uint32_t max2(uint32_t a, uint32_t b) { return a > b ? a : b; }
+  __host__ __device__ static size_t after(size_t at, size_t n) { return (at + n + GAP + 15) / 16 * 16; }
 };
 // Largest segment: two blocks of 2^16-point units (32 768 entries, half as many
 // again in a block 0), four chunks of 1024 points.
 constexpr uint32_t FB_CAP_MAX = 98304;
-static_assert(FB_CAP_MAX / 2 + 3 * FB_GROUP * FB_BUCKETS < 65536, "slot indexes fit 16 bits");
+static_assert(FB_CAP_MAX / 2 + FB_GROUP * FB_BUCKETS + 1 < 65536, "slot indexes fit 16 bits");
 
 __device__ __forceinline__ Fq ld_fq(const Fq* p) {
   const uint4* q = reinterpret_cast<const uint4*>(p);

@@ -271,6 +271,7 @@ struct Lane {
   std::vector<Wd> wd;           // per wide class of the context
   G1Aff* fb_out = nullptr;      // [cap][items][FB_OUT] row and column sums of the bucket grids
   FbScratch fb_scratch;         // k_fb_accum's scratch, one block per persistent CTA
+  bool own_scratch = true;      // freed with the lane (the pipeline's units share one)
   uint32_t* fb_next = nullptr;  // k_fb_accum's item counter
   XYZZ* win = nullptr;          // 8-bit path: [3][L][R][MSM_WINDOWS] (cap 1)
   XYZZ* part = nullptr;         // [cap][3][L][R] per-item MSM results
@@ -292,11 +293,9 @@ struct zg_ctx {
   G1Aff* line_ptr(int c, int l) const { return tab + ((size_t)c * L + l) * W * N; }
   Lane lane;                        // the context's own scratch (one blob slot)
   unsigned fb_ctas[ZG_MSM_PRODUCTS] = {};  // resident CTAs of k_fb_accum per product kind
-  unsigned fb_ctas_max() const {
-    unsigned m = 1;
-    for (unsigned x : fb_ctas) m = std::max(m, x);
-    return m;
-  }
+  // k_fb_accum's scratch for every plan of the context's own lane and of a
+  // pipeline unit (base null)
+  FbScratch lane_scratch, unit_scratch;
   // Wide-window classes (k_wd_sort): class k sorts units of 2^ulog points
   // into 2^ulog buckets of (ulog + 1)-bit digits, for AMT lines l0 .. l0 +
   // nl - 1 (the last one the high line L - 1 when hi_last); tab[c][wl][W][N]
@@ -554,17 +553,111 @@ size_t chunk_offs(const zg_ctx* c) {
 }
 size_t chunk_ents(const zg_ctx* c) { return (size_t)chunk_sets(c).n * 3 * c->N * FB_WINDOWS; }
 
-// k_fb_accum's segment size: the entries of FB_GROUP of a context's largest
-// items, a wide unit's block 0 counted with half as many again, within
-// FB_CAP_MAX
-uint32_t fb_segment(const zg_ctx* c) {
-  uint32_t n = (uint32_t)FB_WINDOWS << std::max(c->lc, FB_UNIT_LOG);
-  for (const zg_ctx::WdClass& k : c->wd) n = std::max(n, ((uint32_t)wd_windows(k.ulog) * 1536u) << k.mlog);
-  return std::min((uint32_t)FB_GROUP * n, FB_CAP_MAX);
+// One item set of a k_fb_accum launch: items, entries of one by its windows and
+// points (no chunk item has more; a wide unit's block 0 up to half as many
+// again, which holds the top window's small digits)
+struct FbSet {
+  uint32_t items, ents;
+  bool wide;
+};
+// Items per CTA and turn of a set in a launch of `units` items: the number g
+// <= `group` that fits a segment of `cap` entries (four fifths of FB_CAP_MAX by
+// the items' usual entries: a group beyond the scratch would run in two
+// segments) and makes rounds x (g entries + FB_TURN_ENTS) smallest, FB_TURN_ENTS
+// being the cost of a turn's chain of inversions in entries at four CTAs per SM.
+// The line is flat: 4 000, 7 000, 12 000 and 18 000 time alike (within 0.5 %)
+// for 64 x 32 to 1024 x 1024 encodes, MSMs of 2^16 to 2^20 and verification.
+constexpr uint32_t FB_TURN_ENTS = 12000;
+uint32_t fb_group_of(const FbSet& k, uint32_t units, uint32_t ctas, uint32_t cap, uint32_t group) {
+  uint64_t best = UINT64_MAX;
+  uint32_t pick = 1;
+  for (uint32_t g = 1; g <= group; ++g) {
+    if (g > 1 && ((uint64_t)g * k.ents * 5 > (uint64_t)FB_CAP_MAX * 4 ||
+                  (uint64_t)g * k.ents * (k.wide ? 5 : 4) > (uint64_t)cap * 4))
+      break;
+    const uint64_t rounds = (units + g * ctas - 1) / (g * ctas);
+    const uint64_t cost = rounds * ((uint64_t)g * (k.ents + 2 * FB_BUCKETS) + FB_TURN_ENTS);
+    if (cost < best) {
+      best = cost;
+      pick = g;
+    }
+  }
+  return pick;
+}
+uint32_t fb_turns(uint32_t items, uint32_t group) { return (items + group - 1) / group; }
+
+// the sets of nb blobs' MSMs with the wide classes in use
+std::vector<FbSet> blob_sets(const zg_ctx* c, int nb) {
+  std::vector<FbSet> r;
+  const ChunkSets cs = chunk_sets(c);
+  for (int b = 0; b < nb; ++b) {
+    for (int k = 0; k < cs.n; ++k)
+      r.push_back(FbSet{chunk_set_items(c, cs.s[k]), (uint32_t)FB_WINDOWS << cs.s[k].ulog, false});
+    for (int k = 0; k < c->wd_on; ++k) {
+      const zg_ctx::WdClass& w = c->wd[k];
+      r.push_back(FbSet{(uint32_t)(3 * (c->R >> w.mlog) * w.nl), ((uint32_t)w.W * FB_BUCKETS) << w.mlog, true});
+    }
+  }
+  return r;
+}
+// enlarges a scratch to what a launch over `sets` takes with each product kind:
+// the segments of the groups it chooses, a block per CTA that gets a turn
+void fb_scratch_for(const zg_ctx* c, const std::vector<FbSet>& sets, FbScratch* s) {
+  uint32_t units = 0;
+  for (const FbSet& k : sets) units += k.items;
+  for (unsigned ctas : c->fb_ctas) {
+    uint32_t turns = 0;
+    for (const FbSet& k : sets) {
+      const uint32_t g = fb_group_of(k, units, ctas, FB_CAP_MAX, FB_GROUP);
+      uint32_t cap = g * k.ents;
+      if (k.wide) cap = std::max(cap / 4 * 5, k.ents / 2 * 3);
+      s->cap = std::max(s->cap, std::min(cap, FB_CAP_MAX));
+      s->group = std::max(s->group, g);
+      turns += fb_turns(k.items, g);
+    }
+    s->ctas = std::max(s->ctas, std::min(ctas, turns));
+  }
+}
+// the single MSMs' item size (zg_ctx_msm above k_fs_accum's sizes): 1024-point
+// chunks leave most SMs idle below 2^19 points (one CTA per item), so chunks
+// shrink down to 128 points until there are 512 items, as far as the context's
+// chunk buffers (3 R chunks) allow; the tables are per point, so any chunking
+// reads them
+int msm_chunk_log(const zg_ctx* c, size_t n) {
+  int lcs = c->lc;
+  while (lcs > 7 && (n >> lcs) < 512 && (n >> (lcs - 1)) <= 3 * c->R) --lcs;
+  return lcs;
+}
+constexpr int FS_MAX_LOG = 15;  // largest single MSM of k_fs_accum, see fs_splits
+// sets c->lane_scratch and c->unit_scratch, for every number of wide classes in
+// use (a tuning choice) and, on the context's own lane, the single MSMs and
+// verification's. Less than a plan would take is still sound: launches choose
+// groups by the scratch, and items beyond `cap` run in segments.
+void plan_scratch(zg_ctx* c) {
+  FbScratch none;
+  none.group = 1;
+  c->lane_scratch = c->unit_scratch = none;
+  const int all = (int)c->wd.size();
+  for (int on = 0; on <= all; ++on) {
+    apply_wide_classes(c, on);
+    fb_scratch_for(c, blob_sets(c, 1), &c->lane_scratch);
+    for (int nb = 1; nb <= FB_MAX_BLOBS; ++nb) fb_scratch_for(c, blob_sets(c, nb), &c->unit_scratch);
+  }
+  for (int k = FS_MAX_LOG + 1; k <= c->lr + c->lc; ++k) {
+    const int lcs = msm_chunk_log(c, (size_t)1 << k);
+    fb_scratch_for(c, {FbSet{1u << (k - lcs), (uint32_t)FB_WINDOWS << lcs, false}}, &c->lane_scratch);
+  }
+  for (uint32_t m = 1; m <= 3; ++m)
+    fb_scratch_for(c, std::vector<FbSet>(m, FbSet{(uint32_t)c->R, (uint32_t)FB_WINDOWS << c->lc, false}), &c->lane_scratch);
+}
+// device bytes of a scratch (k_fs_accum's sums of up to 2^(FS_MAX_LOG - 12)
+// splits use it too)
+size_t scratch_bytes(const FbScratch& s) {
+  return std::max((size_t)s.ctas * s.bytes(), (size_t)(2 * FS_CTAS << std::max(0, FS_MAX_LOG - 12)) * sizeof(XYZZ));
 }
 
-// device bytes of a lane of `cap` blob slots (the request pipeline's
-// admission compares this with the free HBM)
+// device bytes of a lane of `cap` blob slots, its bucket scratch not counted
+// (the request pipeline's admission compares this with the free HBM)
 size_t lane_bytes(const zg_ctx* c, int cap) {
   const size_t N = c->N, R = c->R;
   size_t b = 3 * N * sizeof(Fr);
@@ -577,7 +670,6 @@ size_t lane_bytes(const zg_ctx* c, int cap) {
       if (k.sort_of == (int)j)
         per += 3 * (N >> k.ulog) * (((size_t)1 << k.ulog) + 1) * 4 + 3 * (N >> k.ulog) * wd_unit_ents(k.ulog) * 4;
     }
-    b += (size_t)c->fb_ctas_max() * FbScratch{nullptr, fb_segment(c)}.bytes();
   } else {
     per += 3 * (size_t)c->L * R * MSM_WINDOWS * sizeof(XYZZ);
   }
@@ -585,8 +677,8 @@ size_t lane_bytes(const zg_ctx* c, int cap) {
 }
 
 void free_lane(Lane* ln) {
-  void* ps[] = {ln->T1, ln->Bc, ln->fb_offs, ln->fb_ents, ln->fb_out, ln->fb_scratch.base, ln->fb_next,
-                ln->win, ln->part, ln->nodes};
+  void* ps[] = {ln->T1, ln->Bc, ln->fb_offs, ln->fb_ents, ln->fb_out, ln->own_scratch ? ln->fb_scratch.base : nullptr,
+                ln->fb_next, ln->win, ln->part, ln->nodes};
   for (void* p : ps) if (p) cudaFree(p);
   for (Lane::Wd& w : ln->wd) {
     if (w.offs) cudaFree(w.offs);
@@ -595,7 +687,8 @@ void free_lane(Lane* ln) {
   *ln = Lane();
 }
 
-int alloc_lane(zg_ctx* c, Lane* ln, int cap) {
+// `shared`: a scratch that outlives the lane, or null for one of its own
+int alloc_lane(zg_ctx* c, Lane* ln, int cap, const FbScratch* shared = nullptr) {
   const size_t N = c->N, R = c->R;
   if (cap < 1 || cap > FB_MAX_BLOBS || (!c->fb && cap > 1)) return fail(ZG_ERR_INVALID_ARG, "lane capacity");
   ln->cap = cap;
@@ -613,8 +706,9 @@ int alloc_lane(zg_ctx* c, Lane* ln, int cap) {
       ZG_CK(cudaMalloc(&ln->wd[j].offs, k * 3 * units * (((size_t)1 << c->wd[j].ulog) + 1) * sizeof(uint32_t)));
       ZG_CK(cudaMalloc(&ln->wd[j].ents, k * 3 * units * wd_unit_ents(c->wd[j].ulog) * sizeof(uint32_t)));
     }
-    ln->fb_scratch.cap = fb_segment(c);
-    ZG_CK(cudaMalloc(&ln->fb_scratch.base, (size_t)c->fb_ctas_max() * ln->fb_scratch.bytes()));
+    ln->own_scratch = shared == nullptr;
+    ln->fb_scratch = shared ? *shared : c->lane_scratch;
+    if (!shared) ZG_CK(cudaMalloc(&ln->fb_scratch.base, scratch_bytes(ln->fb_scratch)));
     ZG_CK(cudaMalloc(&ln->fb_next, sizeof(uint32_t)));
   } else {
     ZG_CK(cudaMalloc(&ln->win, 3 * (size_t)c->L * R * MSM_WINDOWS * sizeof(XYZZ)));
@@ -634,6 +728,7 @@ int alloc_blob_buffers(zg_ctx* c) {
     ZG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[3], k_fb_accum<MulW28>, FB_ACC_THREADS, 0));
     ZG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[4], k_fb_accum<MulW28Hybrid>, FB_ACC_THREADS, 0));
     for (int k = 0; k < ZG_MSM_PRODUCTS; ++k) c->fb_ctas[k] = (unsigned)std::max(1, sms * std::max(1, per_sm[k]));
+    plan_scratch(c);
   }
   int rc = alloc_lane(c, &c->lane, 1);
   if (rc) return rc;
@@ -1009,29 +1104,17 @@ __global__ void k_fill_payload(uint8_t* p, uint64_t n, uint64_t seed) {
   }
 }
 
-// Items per CTA and turn of each set: the number g <= FB_GROUP that fits the
-// scratch (four fifths of it by the items' usual entries: a wide unit's block
-// 0 holds up to half as many again, and a group beyond the scratch would run
-// in two segments) and makes rounds x (g entries + FB_TURN_ENTS) smallest,
-// FB_TURN_ENTS being the cost of a turn's chain of inversions (16 of 35 us)
-// in entries at four CTAs per SM. Returns the turns in all.
-constexpr uint32_t FB_TURN_ENTS = 12000;
-uint32_t fb_choose_groups(FbAccPlan& p, uint32_t ctas, uint32_t cap) {
+// Items per CTA and turn of each set (fb_group_of) within a scratch. Returns the
+// turns in all.
+uint32_t fb_choose_groups(FbAccPlan& p, uint32_t ctas, const FbScratch& s) {
   uint32_t turns = 0;
-  const uint32_t units = p.start[p.n];
   for (int k = 0; k < p.n; ++k) {
     FbAccArgs& a = p.a[k];
-    const uint32_t ents = a.ents32 ? ((uint32_t)a.W * FB_BUCKETS) << a.mlog : (uint32_t)FB_WINDOWS << a.lc;
-    uint64_t best = UINT64_MAX;
-    for (uint32_t g = 1; g <= (uint32_t)FB_GROUP && (g == 1 || (uint64_t)g * ents * 5 <= (uint64_t)cap * 4); ++g) {
-      const uint64_t rounds = (units + g * ctas - 1) / (g * ctas);
-      const uint64_t cost = rounds * ((uint64_t)g * (ents + 2 * FB_BUCKETS) + FB_TURN_ENTS);
-      if (cost < best) {
-        best = cost;
-        a.group = (int)g;
-      }
-    }
-    turns += (p.start[k + 1] - p.start[k] + a.group - 1) / a.group;
+    const bool wide = a.ents32 != nullptr;
+    const FbSet set{p.start[k + 1] - p.start[k],
+                    wide ? ((uint32_t)a.W * FB_BUCKETS) << a.mlog : (uint32_t)FB_WINDOWS << a.lc, wide};
+    a.group = (int)fb_group_of(set, p.start[p.n], ctas, s.cap, s.group);
+    turns += fb_turns(set.items, (uint32_t)a.group);
   }
   return turns;
 }
@@ -1040,8 +1123,8 @@ uint32_t fb_choose_groups(FbAccPlan& p, uint32_t ctas, uint32_t cap) {
 // counter and task scratch
 void launch_fb_accum(const zg_ctx* c, const Lane& ln, uint32_t kind, const FbAccPlan& plan, cudaStream_t s) {
   FbAccPlan p = plan;
-  const uint32_t turns = fb_choose_groups(p, c->fb_ctas[kind], ln.fb_scratch.cap);
-  const unsigned grid = std::min<unsigned>(c->fb_ctas[kind], turns);
+  const uint32_t turns = fb_choose_groups(p, c->fb_ctas[kind], ln.fb_scratch);
+  const unsigned grid = std::min({c->fb_ctas[kind], turns, ln.fb_scratch.ctas});
   cudaMemsetAsync(ln.fb_next, 0, sizeof(uint32_t), s);
   auto go = [&](auto kernel) {
     kernel<<<grid, FB_ACC_THREADS, 0, s>>>(p, ln.fb_scratch, ln.fb_next, c->msm_task);
@@ -1126,7 +1209,6 @@ int launch_sum_points(const XYZZ* in, uint32_t n, uint64_t stride, uint32_t sets
 
 // Splits of a single MSM of 2^logn points by k_fs_accum (0: k_fb_accum): 2^12
 // points each, so that a thread sums some 6 entries.
-constexpr int FS_MAX_LOG = 15;
 uint32_t fs_splits(int logn) { return logn > FS_MAX_LOG ? 0 : 1u << std::max(0, logn - 12); }
 
 // the digit sorts of the first `on` wide classes for blob slot b, one launch
@@ -1580,6 +1662,9 @@ struct Engine {
   int fuse = FB_MAX_BLOBS;
   size_t max_units = 3, reserve = 4ull << 30;
   cudaEvent_t last_comp = nullptr;  // compute of the unit issued last (issuer thread only)
+  // k_fb_accum's scratch, one for all units: their computes run one after
+  // another (issue_unit). Allocated with the first unit, by the issuer thread.
+  FbScratch scratch;
   std::thread issuer, recoverer;
 };
 
@@ -1620,14 +1705,23 @@ size_t unit_bytes(const zg_ctx* c, int cap) {
 Unit* make_unit(Engine* e) {
   zg_ctx* c = e->c;
   const int cap = c->fb ? e->fuse : 1;
+  const size_t scratch = c->fb && !e->scratch.base ? scratch_bytes(c->unit_scratch) : 0;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < unit_bytes(c, cap) + e->reserve) {
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < unit_bytes(c, cap) + scratch + e->reserve) {
     cudaGetLastError();
     return nullptr;
   }
+  if (scratch) {
+    FbScratch s = c->unit_scratch;
+    if (cudaMalloc(&s.base, scratch) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    e->scratch = s;
+  }
   std::unique_ptr<Unit> u(new Unit());
   const size_t N = c->N, R = c->R;
-  bool ok = alloc_lane(c, &u->lane, cap) == 0;
+  bool ok = alloc_lane(c, &u->lane, cap, &e->scratch) == 0;
   for (int i = 0; ok && i < cap; ++i) {
     BlobBufs& b = u->b[i];
     ok = cudaMalloc(&b.raw, c->max_blob + 16) == cudaSuccess && cudaMalloc(&b.d_len, 8) == cudaSuccess &&
@@ -1643,6 +1737,10 @@ Unit* make_unit(Engine* e) {
   if (!ok) {
     cudaGetLastError();
     free_unit(u.get());
+    if (e->units.empty() && e->scratch.base) {
+      cudaFree(e->scratch.base);
+      e->scratch = FbScratch();
+    }
     return nullptr;
   }
   return u.release();
@@ -1940,6 +2038,7 @@ void engine_shutdown(Engine* e) {
   }
   for (auto& u : e->units) free_unit(u.get());
   e->units.clear();
+  if (e->scratch.base) cudaFree(e->scratch.base);
   e->c->eng = nullptr;
   delete e;
 }
@@ -3376,14 +3475,8 @@ int zg_ctx_msm(zg_ctx* c, uint32_t coset, uint32_t line, const void* d_scalars, 
   while (((size_t)1 << logn) < n) ++logn;
   const uint32_t splits = fs_splits(logn);
   // Few points: sorted in chunks of up to 1024, XYZZ additions in many short
-  // chains (k_fs_accum). More: work items of 2^lcs points for
-  // k_fb_accum. 1024-point chunks leave most SMs idle below 2^19 points (one
-  // CTA per item), so chunks shrink down to 128 points until there are 512
-  // items, as far as the context's chunk buffers (3 R chunks) allow; the
-  // tables are per point, so any chunking reads them
-  int lcs = splits ? std::min(logn, 10) : c->lc;
-  if (!splits)
-    while (lcs > 7 && (n >> lcs) < 512 && (n >> (lcs - 1)) <= 3 * c->R) --lcs;
+  // chains (k_fs_accum). More: work items of 2^lcs points for k_fb_accum.
+  const int lcs = splits ? std::min(logn, 10) : msm_chunk_log(c, n);
   const int lrn = logn - lcs;
   const uint32_t nch = 1u << lrn;
   std::lock_guard<std::mutex> g(c->mu);

@@ -247,7 +247,7 @@ typedef struct zg_pipeline_stats {
   uint64_t launches[ZG_MAX_FUSED_BLOBS]; /* unit launches of k + 1 blobs */
   uint64_t max_in_flight;     /* most encode requests on the device at once */
   uint64_t recoveries;        /* recovery requests run */
-  uint64_t unit_bytes;        /* device bytes of one unit */
+  uint64_t unit_bytes;        /* device bytes of one unit (the units share one bucket scratch besides) */
 } zg_pipeline_stats;
 int zg_ctx_set_pipeline(zg_ctx* ctx, const zg_pipeline_config* cfg);
 int zg_ctx_pipeline_stats(zg_ctx* ctx, zg_pipeline_stats* out);
