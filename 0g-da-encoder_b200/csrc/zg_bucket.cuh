@@ -310,9 +310,10 @@ struct BktShared {
   }
 };
 // The listings are functions of their own: inlined, they cost the passes
-// registers (a 1024 x 1024 blob of random bytes 107.2 -> 109.2 ms; so 107.7).
+// registers (a 1024 x 1024 blob of random bytes 106.7 -> 108.5 ms; so 107.0).
 // Two pairs are listed at a time, as the stores keep the loads of the next
-// pair behind them (32 x 1024 4.95 -> 4.75 ms).
+// pair behind them (32 x 1024 4.95 -> 4.75 ms), and the counts take the offsets
+// of eight buckets (1024 x 1024 108.0 -> 107.0).
 // Level 1 of entries lo .. hi - 1 of the turn, buckets k0 .. k0 + per - 1 of
 // item `it`, whose first entry is the turn's entry `first` (`mine` false: no
 // such item): lists the pairs, writes what is alone in its bucket, and sets
@@ -345,6 +346,7 @@ static __device__ __noinline__ uint32_t bkt_list_first(BktShared& sh, const BktL
   };
   if (threadIdx.x == 0) sh.runs = 0;  // its last readers are behind a barrier, the next ones behind block_scan's
   uint32_t cnt = 0;  // pairs | slots << 16
+#pragma unroll 8
   for (uint32_t k = k0; k < k0 + per; ++k) {
     const Part p = part(k);
     cnt += ((p.n[0] >> 1) + (p.n[1] >> 1)) + ((((p.n[0] + 1) >> 1) + ((p.n[1] + 1) >> 1) + p.carry) << 16);
@@ -399,6 +401,7 @@ static __device__ __noinline__ uint32_t bkt_list_next(BktShared& sh, uint32_t k0
     return ((uint32_t)sh.sstart[k + 1] - sh.sstart[k] + (1u << lst) - 1) >> (lst + 1);
   };
   uint32_t cnt = 0, np;
+#pragma unroll 8
   for (uint32_t k = k0; k < k0 + per; ++k) cnt += pairs_of(k);
   uint32_t p = block_scan(cnt, sh.wsum, &np);
   for (uint32_t k = k0; k < k0 + per; ++k) {
