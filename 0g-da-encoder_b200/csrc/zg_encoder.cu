@@ -2620,9 +2620,18 @@ extern "C" {
 
 const char* zg_last_error(void) { return g_err.c_str(); }
 
+// The largest shapes of a context, and of one with window tables. k_fb_accum
+// names a table point in 31 bits, the sign on top, and a sort entry's place in
+// 32, over all cosets, lines and windows of a table (a wide class has fewer
+// lines and windows than the 11-bit table).
+constexpr uint32_t MAX_LOG_ROW = 11, MAX_LOG_COL = 11, FB_MAX_LOG_COL = 10;
+static_assert((uint64_t)3 * (MAX_LOG_ROW + 2) * FB_WINDOWS << (MAX_LOG_ROW + FB_MAX_LOG_COL) < uint64_t(1) << 31,
+              "table points fit 31 bits");
+static_assert(wd_windows(WD_MIN_LOG) < FB_WINDOWS && FB_MAX_LOG_COL <= 10, "wide tables are smaller; chunk points fit 10 bits");
+
 int zg_ctx_create(const zg_config* cfg, zg_ctx** out) {
   if (!cfg || !out) return fail(ZG_ERR_INVALID_ARG, "null argument");
-  if (cfg->log_row < 1 || cfg->log_col < 3 || cfg->log_row > 11 || cfg->log_col > 11)
+  if (cfg->log_row < 1 || cfg->log_col < 3 || cfg->log_row > MAX_LOG_ROW || cfg->log_col > MAX_LOG_COL)
     return fail(ZG_ERR_INVALID_ARG, "log_row must be in [1, 11] and log_col in [3, 11]");
   zg_ctx* c = new zg_ctx();
   *out = nullptr;
@@ -2653,7 +2662,7 @@ int zg_ctx_create(const zg_config* cfg, zg_ctx** out) {
   const uint32_t wb = cfg->msm_window_bits;
   if (wb != 0 && wb != 8 && wb != (uint32_t)FB_BITS)
     return bail(fail(ZG_ERR_INVALID_ARG, "msm_window_bits must be 0, 8 or 11"));
-  c->fb = (wb == 0 || wb == (uint32_t)FB_BITS) && c->lc <= 10;
+  c->fb = (wb == 0 || wb == (uint32_t)FB_BITS) && c->lc <= (int)FB_MAX_LOG_COL;
   c->W = c->fb ? FB_WINDOWS : 1;
   if (c->fb && cudaMalloc(&c->tab, (size_t)3 * c->L * c->W * c->N * sizeof(G1Aff)) != cudaSuccess) {
     cudaGetLastError();
