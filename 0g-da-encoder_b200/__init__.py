@@ -256,7 +256,7 @@ def probe_products(device=0, kind="hybrid"):
 def selftest():
     """Mismatch counts of the device arithmetic against its host build."""
     names = ["fq_mul", "fq_mul_f64", "fq_add", "fq_sub", "fr_mul", "fr_roundtrip", "xyzz_dbl", "fq_mul_w28",
-             "fr_mul_f64"]
+             "fr_mul_f64", "fq_inverse", "fr_inverse", "fq_inverse_quad", "quad_add", "quad_dbl"]
     fails = (ctypes.c_int * len(names))()
     _check(lib().zg_selftest(fails, len(names)))
     return dict(zip(names, list(fails)))

@@ -1506,6 +1506,30 @@ __global__ void __launch_bounds__(256) k_ntt_small(Fr* v, int logn, const Fr* tw
 // 4 Fr mul, 5 Fr canonical round trip, 6 XYZZ add vs doubling, 7 Fq mul with
 // 28-bit limbs, 8 Fr mul on the FP64 pipe)
 constexpr int SELFTEST_OPS = 9;
+// then 9 Fq::inverse, 10 Fr::inverse, 11 Fq::inverse_quad against the
+// exponentiation by p - 2, 12 quad_add and 13 quad_dbl against the host's XYZZ
+// formulas
+constexpr int SELFTEST_INV = 3, SELFTEST_CHECKS = SELFTEST_OPS + SELFTEST_INV + 2;
+// values v[i] (below both moduli): res[3 i + {0, 1}] the inverses, [3 i + 2] by
+// thread i's quad; n a multiple of 32
+__global__ void k_selftest_inverse(const Fq* __restrict__ v, Fq* __restrict__ res, uint32_t n) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 4;
+  if (i >= n) return;  // whole warps
+  const Fq q = Fq::inverse_quad(v[i]);
+  if (threadIdx.x & 3) return;
+  res[SELFTEST_INV * i] = v[i].inverse();
+  const Fr r = reinterpret_cast<const Fr*>(v)[i].inverse();
+  res[SELFTEST_INV * i + 1] = *reinterpret_cast<const Fq*>(&r);
+  res[SELFTEST_INV * i + 2] = q;
+}
+// sums and doublings of points by quads, eight pairs a warp; n a multiple of 8
+__global__ void k_selftest_quad(const XYZZ* __restrict__ a, const XYZZ* __restrict__ b, XYZZ* __restrict__ res, uint32_t n) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 4;
+  if (i >= n) return;  // whole warps
+  const Fq x = quad_load(a + i);
+  quad_store(res + 2 * i, quad_add(x, quad_load(b + i)));
+  quad_store(res + 2 * i + 1, quad_dbl(x));
+}
 __global__ void k_selftest(const Fq* a, const Fq* b, Fq* res, uint32_t n) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -3659,6 +3683,103 @@ int zg_ntt(void* d_data, uint32_t log_n, uint32_t batch, int inverse, uint32_t c
 }
 
 
+namespace {
+// checks 9 .. 13: inverses of edge values and random ones, quad sums with
+// equal, opposite and infinite points in any quads of a warp
+int selftest_curve(int* fails) {
+  std::vector<Fq> v;
+  auto put = [&](Fq x) {  // below both moduli
+    Fq d;
+    if (Fr::sub_raw(*reinterpret_cast<Fr*>(&d), *reinterpret_cast<Fr*>(&x), Fr::modulus())) v.push_back(x);
+  };
+  for (int k = 0; k < 256; ++k) {
+    Fq x = Fq::zero();
+    x.v[k / 32] = 1u << (k % 32);
+    put(x);
+    put(-x);
+    Fr r = -*reinterpret_cast<Fr*>(&x);
+    put(*reinterpret_cast<Fq*>(&r));
+  }
+  put(Fq::zero());
+  uint64_t st = 0x9876;
+  while (v.size() < 2048) {
+    Fq x;
+    for (int k = 0; k < 8; ++k) x.v[k] = (uint32_t)splitmix64(st);
+    x.v[7] &= v.size() & 1 ? 0x3fffffffu : 0xffu;
+    put(x);
+  }
+  const uint32_t n = (uint32_t)v.size();
+  // multiples of the generator, each with a ZZ of its own
+  std::vector<XYZZ> a(n), b(n);
+  XYZZ g = XYZZ::from_affine(G1Aff{Fq::from_u32(1), Fq::from_u32(2)}), p = g;
+  auto scaled = [&](const XYZZ& q) {
+    Fq z;
+    for (int k = 0; k < 8; ++k) z.v[k] = (uint32_t)splitmix64(st);
+    z.v[7] &= 0x0fffffffu;
+    const Fq zz = z * z, zzz = zz * z;
+    XYZZ r = q;
+    r.X = q.X * zz;
+    r.Y = q.Y * zzz;
+    r.ZZ = q.ZZ * zz;
+    r.ZZZ = q.ZZZ * zzz;
+    return r;
+  };
+  for (uint32_t i = 0; i < n; ++i) {
+    p.add(g);
+    a[i] = scaled(p);
+    b[i] = scaled(i ? a[i - 1] : g);
+    const uint64_t kind = splitmix64(st) % 8;  // any mixture within a warp
+    if (kind == 0) b[i] = scaled(p);
+    if (kind == 1) {
+      b[i] = scaled(p);
+      b[i].Y = -b[i].Y;
+    }
+    if (kind == 2) a[i] = XYZZ::inf();
+    if (kind == 3) b[i] = XYZZ::inf();
+    if (kind == 4 && i % 3 == 0) a[i] = b[i] = XYZZ::inf();
+  }
+  Fq *dv = nullptr, *dr = nullptr;
+  XYZZ *da = nullptr, *db = nullptr, *ds = nullptr;
+  ZG_CK(cudaMalloc(&dv, n * sizeof(Fq)));
+  ZG_CK(cudaMalloc(&dr, SELFTEST_INV * n * sizeof(Fq)));
+  ZG_CK(cudaMalloc(&da, n * sizeof(XYZZ)));
+  ZG_CK(cudaMalloc(&db, n * sizeof(XYZZ)));
+  ZG_CK(cudaMalloc(&ds, 2 * n * sizeof(XYZZ)));
+  ZG_CK(cudaMemcpy(dv, v.data(), n * sizeof(Fq), cudaMemcpyHostToDevice));
+  ZG_CK(cudaMemcpy(da, a.data(), n * sizeof(XYZZ), cudaMemcpyHostToDevice));
+  ZG_CK(cudaMemcpy(db, b.data(), n * sizeof(XYZZ), cudaMemcpyHostToDevice));
+  k_selftest_inverse<<<n / 32, 128>>>(dv, dr, n);
+  k_selftest_quad<<<n / 32, 128>>>(da, db, ds, n);
+  ZG_CK(cudaDeviceSynchronize());
+  std::vector<Fq> r(SELFTEST_INV * n);
+  std::vector<XYZZ> s(2 * n);
+  ZG_CK(cudaMemcpy(r.data(), dr, r.size() * sizeof(Fq), cudaMemcpyDeviceToHost));
+  ZG_CK(cudaMemcpy(s.data(), ds, s.size() * sizeof(XYZZ), cudaMemcpyDeviceToHost));
+  for (void* x : {(void*)dv, (void*)dr, (void*)da, (void*)db, (void*)ds}) cudaFree(x);
+  Fq two = Fq::zero(), eq, er;
+  two.v[0] = 2;
+  Fq::sub_raw(eq, Fq::modulus(), two);
+  Fr::sub_raw(*reinterpret_cast<Fr*>(&er), Fr::modulus(), *reinterpret_cast<Fr*>(&two));
+  auto same = [](const XYZZ& x, const XYZZ& y) {
+    G1Aff e, f;
+    const bool fx = x.to_affine(e), fy = y.to_affine(f);
+    return fx == fy && (!fx || (e.x == f.x && e.y == f.y));
+  };
+  for (uint32_t i = 0; i < n; ++i) {
+    const Fq inv = v[i].pow(eq.v, 8);
+    const Fr rinv = reinterpret_cast<Fr*>(&v[i])->pow(er.v, 8);
+    fails[0] += r[SELFTEST_INV * i] != inv;
+    fails[1] += r[SELFTEST_INV * i + 1] != *reinterpret_cast<const Fq*>(&rinv);
+    fails[2] += r[SELFTEST_INV * i + 2] != inv;
+    XYZZ sum = a[i];
+    sum.add(b[i]);
+    fails[3] += !same(s[2 * i], sum);
+    fails[4] += !same(s[2 * i + 1], a[i].dbl());
+  }
+  return ZG_OK;
+}
+}  // namespace
+
 int zg_selftest(int* fails, int nops) {
   const uint32_t n = 1024;
   std::vector<Fq> a(n), b(n);
@@ -3711,6 +3832,11 @@ int zg_selftest(int* fails, int nops) {
     for (int k = 0; k < SELFTEST_OPS; ++k) cnt[k] += (r[SELFTEST_OPS * i + k] != e[k]);
   }
   for (int k = 0; k < nops && k < SELFTEST_OPS; ++k) fails[k] = cnt[k];
+  if (nops <= SELFTEST_OPS) return ZG_OK;
+  int more[SELFTEST_CHECKS - SELFTEST_OPS] = {};
+  const int rc = selftest_curve(more);
+  if (rc) return rc;
+  for (int k = SELFTEST_OPS; k < nops && k < SELFTEST_CHECKS; ++k) fails[k] = more[k - SELFTEST_OPS];
   return ZG_OK;
 }
 
