@@ -47,7 +47,8 @@ bool host_parallel(size_t n, size_t grain, size_t most, F fn) {
 // of rows and 4 MB of payload of a 128 x 1024 recovery take 1.77 ms with one
 // thread, 1.80, 1.91, 2.02 and 2.57 with 2, 4, 8 and 16 (12.6 MB: 2.32, 2.23,
 // 2.18, 2.44, 2.87); 50 and 32 MB of a 1024 x 1024 one 20.9, 17.5, 15.6, 13.3
-// and 14.0 ms (a B200 host of 16 cores).
+// and 14.0 ms (a B200 host of 16 cores; calls that zero-filled a buffer for the
+// result and copied it once more: without that 1.37, 1.90 and 8.3 ms).
 constexpr size_t COPY_SERIAL_BELOW = size_t(16) << 20;
 constexpr size_t COPY_THREADS = 8;
 inline size_t copy_threads(size_t bytes) { return bytes < COPY_SERIAL_BELOW ? 1 : COPY_THREADS; }
