@@ -12,7 +12,9 @@
 // same), so the product is bounded by 128 wide + 8 narrow multiply-adds = 4.1
 // clocks per SM; measured 4.5 (64 G products/s on a B200, multiply pipe 92 %
 // busy), against 6.1 clocks (47 G/s) for one accumulator array, whose odd
-// chains straddle the pairs and issue lo and hi apart. Outputs that are
+// chains straddle the pairs and issue lo and hi apart. (Separate rows for even
+// and odd limbs are a published technique of big-number libraries for GPUs
+// with multiply-adds on register pairs.) Outputs that are
 // written before every input of an asm block has been read are early-clobber
 // ("=&r"), so the compiler never assigns them an input's register. Host builds
 // use a portable 64-bit path with identical results.

@@ -9,7 +9,9 @@
 //    double;
 //  * a limb product xy (< 2^102) is split exactly into hi = floor(xy / 2^51)
 //    and lo = xy mod 2^51 by two FMAs: h = fma_rz(x, y, 2^103) holds hi in its
-//    mantissa, and l = fma(x, y, 2^103 + 2^52 - h) = 2^52 + lo is exact;
+//    mantissa, and l = fma(x, y, 2^103 + 2^52 - h) = 2^52 + lo is exact (the
+//    split of Emmart, Zheng and Weems, "Faster Modular Exponentiation Using
+//    Double Precision Floating Point Arithmetic on the GPU", ARITH 2018);
 //  * two products of one column share their sums: the second's FMA starts
 //    from the first's h (2^103 + two halves < 2^104, the same binade), and the
 //    two low halves meet in one FP64 addition (2^52 + lo + lo' < 2^53);

@@ -483,9 +483,9 @@ __global__ void __launch_bounds__(MSM_THREADS, 1) k_msm_chunks(MsmChunkArgs a) {
 // stored with its window multiples T_w = 2^{11 w} P (w < 24): a chunk MSM
 //   sum_t s_t P_t = sum_t sum_w d_{t,w} T_w[t]
 // over the signed 11-bit digits d of the scalars is one bucket accumulation
-// (buckets |d| = 1..1024) with no doublings. Per chunk: ~24 x 1024 mixed adds
-// plus 2 x 1024 bucket-reduction adds, against 32 x (1024 + 256) for 8-bit
-// windows with doublings.
+// (buckets |d| = 1..1024) with no doublings. Per chunk: ~24 x 1024 affine
+// additions, 2 x 31 x 32 of the bucket grid and 126 XYZZ ones of the combine,
+// against 32 x (1024 + 256) for 8-bit windows with doublings.
 constexpr int FB_BITS = 11;
 constexpr int FB_WINDOWS = 24;                    // ceil((254 + 1) / 11)
 constexpr int FB_BUCKETS = 1 << (FB_BITS - 1);    // 1024
@@ -582,7 +582,7 @@ __device__ __forceinline__ uint32_t fb_window_bits(const uint32_t* s, int w) {
 constexpr int FB_MAX_CHUNK_SETS = 8;  // sets of 11-bit items of a blob (more than one: no wide classes)
 // The units that one k_fb_sort launch sorts: set k's blocks start[k] ..
 // start[k + 1] - 1 take the units of 2^ulog[k] points of one vector per
-// blockIdx.y, units[k] per vector
+// blockIdx.y
 struct FbSortPlan {
   int n = 0;
   uint32_t start[FB_MAX_CHUNK_SETS + 1] = {};
@@ -965,8 +965,8 @@ __global__ void __launch_bounds__(128) k_fb_combine_warp(const G1Aff* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// A single MSM over few points, where k_fb_accum's chain of tree levels and
-// shared inversions (30 us each) is the time: the chunks' sorted lists
+// A single MSM over few points, where k_fb_accum's chain of tree levels, one
+// shared inversion (14 us) each, is the time: the chunks' sorted lists
 // (k_fb_sort) share one set of buckets, cut into groups of FS_BUCKETS, one CTA
 // of 128 threads per group and split. XYZZ additions: each thread sums the
 // entries of an even share of its group's list, the threads' partial sums of
@@ -975,9 +975,9 @@ __global__ void __launch_bounds__(128) k_fb_combine_warp(const G1Aff* __restrict
 // digits are 0, 1 or 2 (scalars below r), so its entries in buckets 0 and 1
 // (half the points) go to FS_TOP extra CTAs per split instead of making group
 // 0 the last to finish.
-// Whole MSM of 2^10 / 2^12 / 2^14 / 2^15 points: 0.23 / 0.36 / 0.50 / 0.73 ms,
-// against 0.75 / 0.75 / 0.76 / 0.93 by k_fb_accum; from 2^16 on the affine
-// additions win (1.24 against 1.47 ms at 2^16).
+// Whole MSM of 2^10 / 2^12 / 2^14 / 2^15 points: 0.235 / 0.374 / 0.50 / 0.72 ms,
+// against 0.64 / 0.64 / 0.65 / 0.73 by k_fb_accum; from 2^16 on the affine
+// additions win (1.04 against 1.25 ms at 2^16, 1.30 against 2.27 at 2^17).
 constexpr int FS_BUCKETS = 8;
 constexpr int FS_GROUPS = FB_BUCKETS / FS_BUCKETS;  // 128
 constexpr int FS_TOP = 16;                          // CTAs for the top window, per split
